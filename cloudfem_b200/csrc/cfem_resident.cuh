@@ -1,0 +1,874 @@
+// Resident PCG: every phase of a solve in one cooperative launch, with one
+// block per SM and a fixed share of a system's rows per block. Included by
+// cfem_solve.cu (it uses that file's SysDev, SysState, advance()).
+//
+// What bounds a CG iteration on the systems this runs is not traffic but
+// the chain of dependent steps - gathers, block sums, the grid-wide sum and
+// the scalars that follow from it - and the L1 throughput of 32-way
+// scattered gathers. So a block keeps what it alone reads in shared memory
+// for the whole solve: its rows' vectors, as many of its matrix slices as
+// fit (the 148 SMs hold 33 MB between them; the rest streams from L2 or
+// HBM), and the part of the direction that its rows' columns name (the
+// halo). The product phase first loads the halo, every distinct column once
+// and all of them in flight together, and then gathers from shared memory
+// with 16-bit local columns.
+//
+// The grid meets twice per iteration in a sum that is its own barrier: every
+// block writes its partial sums with an epoch in one 16-byte word, one warp
+// of every block reads all the words, adds them in block order and advances
+// the system's state for its own block. No atomics, and no second round trip
+// to fetch the result. The words are kept in several copies, each read by
+// its share of the blocks: 148 blocks polling one copy took 10.0 us for an
+// iteration's two sums (measured without the CG arithmetic), 8 copies 6.7 us.
+//
+// A neighbour's z and its previous direction p, from which the new direction
+// p = zeta z + beta p follows, are stored as pairs, so the halo is one load
+// per entry. A pair is written by its row's block in the update phase and
+// read in the product phase, with the grid's sum between them.
+//
+// Measured per iteration (residual replacements included), before on the
+// launches over CSR or on the graph scheduler, and here: P1 box 20^3 in FP64
+// 22 -> 7.2 us; Tet10 cantilever of 40 x 5 x 5 cells in FP64 41 -> 10.7 us
+// (0.6 halo, 1.8 products, 3.2 sum, 0.4 update, 4.3 sum); Tet10 box of 27 x
+// 15 x 13 cells, elasticity in FP32, 52 MB of blocks of which 60 % fit, 32
+// -> 19 us; Tet10 heat of 44,415 rows in FP32 45 -> 10.0 us; P1 heat of
+// 699,273 rows in FP64 (104 MB streamed per iteration at 5.2 TB/s) 60 -> 43 us.
+//
+// Sums depend on the system's own shape (block count, rows per block, lanes
+// per row), never on what else is in the batch, so a result is bitwise the
+// same alone and in a batch.
+
+constexpr int RT = 512;              // threads per block
+constexpr int RWARPS = RT / 32;
+constexpr int RS_WINDOW = 256;       // rows sorted by length together
+constexpr int RS_SMEM_MAX = 224 * 1024;
+constexpr size_t RS_MAX_WAVES = 4;   // launches of one batch
+constexpr int RS_COPIES = 8;         // copies of the partial sums, at most
+
+template <typename T> struct PairOf;
+template <> struct PairOf<float> { using type = float2; };
+template <> struct PairOf<double> { using type = double2; };
+
+// A block of the batch: its system, its number there, its rows and its
+// first slice in the batch's slice table.
+struct RsCta {
+    int32_t sys, cta, row0, rows;
+    int64_t sl0;
+};
+
+struct RsShared {
+    double red[4][RWARPS];
+    SysState st;
+    int quit;
+    int nres;                        // leading slices held in shared memory
+    int own;                         // place of the block's first row in its halo
+};
+
+__host__ __device__ inline size_t rs_al(size_t v) { return (v + 15) & ~(size_t)15; }
+__host__ __device__ inline int rs_slices(int rows, int lsh) {   // of 32 / L rows
+    return (rows + (32 >> lsh) - 1) >> (5 - lsh);
+}
+// Shared-memory bytes of a block's slice offsets and row order, of its halo
+// (column list and direction) and of its rows' vectors (q, r, the Jacobi
+// inverse and the fixed mask).
+__host__ __device__ inline size_t rs_meta_bytes(int rows, int lsh) {
+    const size_t nsl = (size_t)rs_slices(rows, lsh);
+    return rs_al((nsl + 1) * 4) + rs_al(nsl << (5 - lsh));
+}
+__host__ __device__ inline size_t rs_halo_bytes(int u, int bs, size_t ts) {
+    return rs_al((size_t)u * 4) + rs_al((size_t)u * bs * ts);
+}
+__host__ __device__ inline size_t rs_vec_bytes(int rows, int bs, size_t ts) {
+    const size_t nd = (size_t)rows * bs;
+    return 3 * rs_al(nd * ts) + rs_al(nd);
+}
+// Copies of the words: contention grows with the blocks that poll one.
+__host__ __device__ inline int rs_copies_of(int ncta) {
+    return ncta > 24 ? RS_COPIES : (ncta > 4 ? 4 : 1);
+}
+__host__ __device__ inline size_t rs_mail_bytes(int ncta) {
+    return (size_t)2 * 4 * rs_copies_of(ncta) * ncta * sizeof(ulonglong2);
+}
+
+__device__ __forceinline__ uint16_t ld_stream(const uint16_t *p) {
+    uint16_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+
+// One block's partial sum of one quantity: the value and the epoch it
+// belongs to in one 16-byte word that is written and read whole.
+__device__ __forceinline__ void mail_put(ulonglong2 *p, double v, unsigned long long epoch) {
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\t"
+                 "st.relaxed.gpu.global.b128 [%0], t;\n\t}"
+                 :: "l"(p), "l"(__double_as_longlong(v)), "l"(epoch) : "memory");
+}
+__device__ __forceinline__ bool mail_get(const ulonglong2 *p, unsigned long long epoch, double &v) {
+    long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\t"
+                 "mov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    v = __longlong_as_double(lo);
+    return (unsigned long long)hi == epoch;
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Grid-wide sum of NV quantities over the system's blocks, then the state
+// transition, in every block for itself. PUB: what the block wrote to
+// global memory before is visible to the system's other blocks after it,
+// and theirs to this one (the product phase writes nothing others read and
+// goes without). Returns false when a block gave up waiting (bounded:
+// timeout_ns).
+template <int NV, bool PUB>
+__device__ __forceinline__ bool rs_sync(const SysDev &S, RsShared &sh, GridBar *bar, int cta,
+                                        int ph, unsigned long long epoch, double part[4],
+                                        unsigned long long timeout_ns, unsigned hold) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) part[v] = warp_sum(part[v]);
+    if (lane == 0)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) sh.red[v][w] = part[v];
+    __syncthreads();
+    if (w == 0) {
+        double tot[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            double t = sh.red[v][lane & (RWARPS - 1)];
+#pragma unroll
+            for (int o = RWARPS / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            tot[v] = t;
+        }
+        bool ok = true;
+        if (S.ncta > 1 || hold) {
+            const int nc = S.ncta, R = rs_copies_of(nc);
+            // two sets of words in turn: a block writes set e + 2 only after
+            // every block has written, and so read past, set e
+            ulonglong2 *box = S.mail + (size_t)(epoch & 1) * 4 * R * nc;
+            if (PUB) fence_gpu();    // the block's writes before its words
+            if (lane < R)
+#pragma unroll
+                for (int v = 0; v < NV; ++v)
+                    mail_put(box + (size_t)(4 * lane + v) * nc + cta, tot[v], epoch);
+            const ulonglong2 *in = box + (size_t)4 * (cta % R) * nc;
+            constexpr int PER = (RS_MAX_CTAS + 31) / 32;
+            double got[NV][PER];
+            unsigned long long t0 = 0;
+            for (unsigned spin = 0;; ++spin) {
+                bool all = hold == 0;
+#pragma unroll
+                for (int v = 0; v < NV; ++v)
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) {
+                        const int c = lane + 32 * k;
+                        got[v][k] = 0.0;
+                        if (c < nc) all &= mail_get(in + v * nc + c, epoch, got[v][k]);
+                    }
+                if (__all_sync(0xffffffffu, all)) break;
+                if ((spin & 63u) == 63u) {
+                    const unsigned long long now = globaltimer();
+                    if (t0 == 0) t0 = now;
+                    int stop = 0;
+                    if (lane == 0) {
+                        if (now - t0 > timeout_ns) atomicExch(&bar->err, 1);
+                        stop = *(volatile int *)&bar->err;
+                    }
+                    if (__shfl_sync(0xffffffffu, stop, 0)) {
+                        ok = false;
+                        break;
+                    }
+                }
+            }
+            if (PUB) fence_gpu();    // the other blocks' writes after their words
+            if (ok)
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    double t = 0.0;
+#pragma unroll
+                    for (int k = 0; k < PER; ++k) t += got[v][k];
+                    tot[v] = warp_sum(t);
+                }
+        }
+        if (lane == 0) {
+            if (!ok) {
+                sh.quit = 1;
+            } else {
+                if (ph == PH_INIT && tot[3] < 0.0) sh.st.status = CFEM_ERR_BREAKDOWN;
+                advance(S, &sh.st, bar, ph, tot, cta == 0);
+            }
+        }
+    }
+    __syncthreads();
+    return sh.quit == 0;
+}
+
+// U steps of one slice from step t on, loaded together; steps past the
+// slice's last repeat it with coefficient 0.
+template <typename T, int U, bool SM>
+__device__ __forceinline__ void rs_load(const uint16_t *cp, const T *vp, int t, int w, int c[U],
+                                        T a[U]) {
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const int tt = t + j < w ? t + j : w - 1;
+        c[j] = SM ? cp[32 * tt] : ld_stream(cp + 32 * tt);
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        const int tt = t + j < w ? t + j : w - 1;
+        a[j] = SM ? vp[32 * tt] : ld_stream(vp + 32 * tt);
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) a[j] = t + j < w ? a[j] : (T)0;
+}
+
+// One lane's part of a row of a slice of 32 / L rows (L lanes per row):
+// slot k of a row sits at step k / L in lane k % L of the row's lanes; slot
+// 0 (diag: this lane holds it) is the diagonal, or the row sum of the FP32
+// difference form (DIFF), whose other slots multiply p_j - p_i.
+template <typename T, bool DIFF, int U, bool SM>
+__device__ __forceinline__ T rs_steps1(const uint16_t *cp, const T *vp, int t, int w, bool diag,
+                                       const T *halo, T pi) {
+    int c[U];
+    T a[U];
+    rs_load<T, U, SM>(cp, vp, t, w, c, a);
+    T acc = 0;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+        T pj = halo[c[j]];
+        if (DIFF) pj = (diag && t + j == 0) ? pi : pj - pi;
+        acc += a[j] * pj;
+    }
+    return acc;
+}
+
+template <typename T, bool DIFF, bool SM>
+__device__ __forceinline__ T rs_row1(const uint16_t *cp, const T *vp, int w, bool diag,
+                                     const T *halo, T pi) {
+    T acc = 0;
+    int t = 0;
+    for (; w - t > 4; t += 8) acc += rs_steps1<T, DIFF, 8, SM>(cp, vp, t, w, diag, halo, pi);
+    if (t < w) acc += rs_steps1<T, DIFF, 4, SM>(cp, vp, t, w, diag, halo, pi);
+    return acc;
+}
+
+// The same over 3x3 blocks: nine value planes of 32 lanes per step.
+template <typename T, bool DIFF, bool SM>
+__device__ __forceinline__ void rs_row3(const uint16_t *cp, const T *vp, int w, bool diag,
+                                        const T *halo, const T pi[3], T acc[3]) {
+    constexpr int U = !SM && sizeof(T) == 4 ? 4 : 2;
+    for (int t = 0; t < w; t += U) {
+        int c[U];
+        T a[U][9];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int tt = t + j < w ? t + j : w - 1;
+            c[j] = SM ? cp[32 * tt] : ld_stream(cp + 32 * tt);
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int tt = t + j < w ? t + j : w - 1;
+#pragma unroll
+            for (int e = 0; e < 9; ++e)
+                a[j][e] = SM ? vp[32 * (9 * tt + e)] : ld_stream(vp + 32 * (9 * tt + e));
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            T pj[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                pj[d] = halo[3 * c[j] + d];
+                if (DIFF) pj[d] = (diag && t + j == 0) ? pi[d] : pj[d] - pi[d];
+                if (t + j >= w) pj[d] = 0;
+            }
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) acc[r] += a[j][r * 3 + d] * pj[d];
+        }
+    }
+}
+
+// Compensated sums of one lane's part of a row for the FP64 true residual
+// (x in the halo), with the sum of magnitudes for its round-off floor.
+template <int BS, bool SM>
+__device__ __forceinline__ void rs_row_dd(const uint16_t *cp, const double *vp, int w,
+                                          const double *halo, double hi[BS], double lo[BS],
+                                          double ab[BS]) {
+    constexpr int B2 = BS * BS, U = BS == 1 ? 4 : 1;
+    for (int t = 0; t < w; t += U) {
+        int c[U];
+        double a[U][B2];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int tt = t + j < w ? t + j : w - 1;
+            c[j] = SM ? cp[32 * tt] : ld_stream(cp + 32 * tt);
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int tt = t + j < w ? t + j : w - 1;
+#pragma unroll
+            for (int e = 0; e < B2; ++e)
+                a[j][e] = SM ? vp[32 * (B2 * tt + e)] : ld_stream(vp + 32 * (B2 * tt + e));
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            if (t + j >= w) continue;
+#pragma unroll
+            for (int d = 0; d < BS; ++d) {
+                const double xj = halo[BS * c[j] + d];
+#pragma unroll
+                for (int r = 0; r < BS; ++r) {
+                    dd_fma(hi[r], lo[r], a[j][r * BS + d], xj);
+                    ab[r] += fabs(a[j][r * BS + d] * xj);
+                }
+            }
+        }
+    }
+}
+
+template <typename T, int BS>
+__global__ void __launch_bounds__(RT, 1)
+k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
+           const RsCta *__restrict__ ctas, int first_cta, const int2 *__restrict__ ucnt,
+           const int32_t *__restrict__ ulist, int umax, const uint16_t *__restrict__ scol,
+           const T *__restrict__ sval, int nbytes, int vsm, int max_steps,
+           unsigned long long timeout_ns, unsigned hold) {
+    extern __shared__ __align__(128) unsigned char rs_area[];
+    __shared__ RsShared sh;
+    __shared__ SysDev S;
+    using P2 = typename PairOf<T>::type;
+    constexpr bool DIFF = sizeof(T) == 4;
+    constexpr int B2 = BS * BS;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int gcta = first_cta + blockIdx.x;
+    const RsCta me = ctas[gcta];
+    const int cta = me.cta;
+    for (int i = tid; i < (int)(sizeof(SysDev) / 4); i += RT)
+        ((int *)&S)[i] = __ldg((const int *)(sys + me.sys) + i);
+    if (tid == 0) {
+        memset(&sh.st, 0, sizeof(SysState));
+        sh.quit = 0;
+        sh.own = 0;
+    }
+    __syncthreads();
+    const int lsh = S.lsh, L = 1 << lsh;
+    const int nloc = me.rows, nd = nloc * BS, nsl = rs_slices(nloc, lsh);
+    const int64_t r0 = me.row0, d0 = r0 * BS;
+    P2 *pair = (P2 *)S.pair;
+    const int nu = __ldg(&ucnt[gcta].x);
+    // the block's own arrays
+    unsigned char *area = rs_area;
+    int *so = (int *)area;                       // slice offsets, from the block's first
+    area += rs_al((size_t)(nsl + 1) * 4);
+    uint8_t *perm = area;
+    area += rs_al((size_t)nsl << (5 - lsh));
+    int32_t *list = (int32_t *)area;
+    area += rs_al((size_t)nu * 4);
+    T *halo = (T *)area;
+    area += rs_al((size_t)nu * BS * sizeof(T));
+    T *q, *r, *dinv;
+    const uint8_t *fx;
+    if (vsm) {
+        const size_t one = rs_al((size_t)nd * sizeof(T));
+        q = (T *)area;
+        r = (T *)(area + one);
+        dinv = (T *)(area + 2 * one);
+        uint8_t *f = area + 3 * one;
+        for (int i = tid; i < nd; i += RT) f[i] = S.fixed ? __ldg(S.fixed + d0 + i) : 0;
+        fx = f;
+        area += rs_vec_bytes(nloc, BS, sizeof(T));
+    } else {
+        q = (T *)S.q + d0;
+        r = (T *)S.r + d0;
+        dinv = (T *)S.dinv + d0;
+        fx = S.fixed ? S.fixed + d0 : nullptr;
+    }
+    const int64_t *gso = S.soff + me.sl0;
+    const int64_t off0 = __ldg(gso);
+    for (int i = tid; i <= nsl; i += RT) so[i] = (int)(__ldg(gso + i) - off0);
+    for (int i = tid; i < nsl << (5 - lsh); i += RT)
+        perm[i] = __ldg(S.sperm + me.sl0 * 32 + i);
+    for (int i = tid; i < nu; i += RT) {
+        const int32_t c = __ldg(ulist + (size_t)gcta * umax + i);
+        list[i] = c;
+        if (c == (int32_t)r0) sh.own = i;        // own rows follow one another in the list
+    }
+    __syncthreads();
+    // as many of the leading slices as fit
+    const size_t cost = 2 + B2 * sizeof(T);
+    const size_t room = (size_t)nbytes - (size_t)(area - rs_area);
+    if (tid == 0) {
+        int lo = 0, hi = nsl;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if ((size_t)so[mid] * cost <= room) lo = mid; else hi = mid - 1;
+        }
+        sh.nres = lo;
+    }
+    __syncthreads();
+    const int nres = sh.nres;
+    const int eres = so[nres];                   // entries held (a multiple of 32)
+    T *mv = (T *)area;
+    uint16_t *mc = (uint16_t *)(area + (size_t)eres * B2 * sizeof(T));
+    const uint16_t *gc = scol + off0;
+    const T *gv = sval + (size_t)B2 * off0;
+    {
+        const int n16 = (int)((size_t)eres * B2 * sizeof(T) / 16);
+        for (int i = tid; i < n16; i += RT) ((int4 *)mv)[i] = __ldcs((const int4 *)gv + i);
+        for (int i = tid; i < eres / 8; i += RT) ((int4 *)mc)[i] = __ldcs((const int4 *)gc + i);
+    }
+    const T *pown = halo + (size_t)sh.own * BS;  // the direction on the block's own rows
+    __syncthreads();
+
+    int ph = PH_INIT;
+    unsigned long long epoch = 0;
+    for (int step = 0; step < max_steps; ++step) {
+        double part[4] = {0.0, 0.0, 0.0, 0.0};
+        ++epoch;
+        bool ok;
+        if (ph == PH_A) {
+            const T beta = (T)sh.st.beta, zeta = (T)sh.st.zeta;
+            const int nh = nu * BS;
+            for (int i0 = tid; i0 < nh; i0 += 4 * RT) {
+                P2 g[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = i0 + k * RT < nh ? i0 + k * RT : i0;
+                    const int e = BS == 1 ? i : i / 3;
+                    g[k] = __ldcg(pair + (int64_t)BS * list[e] + (BS == 1 ? 0 : i - 3 * e));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i0 + k * RT < nh) halo[i0 + k * RT] = zeta * g[k].x + beta * g[k].y;
+            }
+            __syncthreads();
+            double pq = 0.0;
+            const int grp = lane >> lsh;
+            const bool first = (lane & (L - 1)) == 0;
+            for (int s = wid; s < nsl; s += RWARPS) {
+                const int off = so[s], w = (so[s + 1] - off) >> 5;
+                const int pos = s * (32 >> lsh) + grp;
+                const int rl = (pos & ~(RS_WINDOW - 1)) + perm[pos];
+                const bool valid = rl < nloc;
+                const int ri = valid ? rl : 0;
+                T pi[BS], acc[BS];
+#pragma unroll
+                for (int c = 0; c < BS; ++c) {
+                    pi[c] = pown[ri * BS + c];
+                    acc[c] = 0;
+                }
+                if constexpr (BS == 1) {
+                    acc[0] = s < nres ? rs_row1<T, DIFF, true>(mc + off + lane, mv + off + lane, w, first,
+                                                               halo, pi[0])
+                                      : rs_row1<T, DIFF, false>(gc + off + lane, gv + off + lane, w, first,
+                                                                halo, pi[0]);
+                } else {
+                    if (s < nres)
+                        rs_row3<T, DIFF, true>(mc + off + lane, mv + 9 * (size_t)off + lane, w, first,
+                                               halo, pi, acc);
+                    else
+                        rs_row3<T, DIFF, false>(gc + off + lane, gv + 9 * (size_t)off + lane, w, first,
+                                                halo, pi, acc);
+                }
+                for (int o = L >> 1; o > 0; o >>= 1)
+#pragma unroll
+                    for (int c = 0; c < BS; ++c) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+                if (valid && first) {
+#pragma unroll
+                    for (int c = 0; c < BS; ++c) {
+                        q[rl * BS + c] = acc[c];
+                        pq += (double)pi[c] * (double)acc[c];
+                    }
+                }
+            }
+            part[0] = pq;
+            ok = rs_sync<1, false>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+        } else if (ph == PH_B) {
+            const double alpha64 = sh.st.alpha;
+            const T alpha = (T)alpha64;
+            double rz = 0.0, rr = 0.0;
+            double *x = S.x + d0;
+            for (int i = tid; i < nd; i += RT) {
+                const bool fixed = fx && fx[i];
+                const T pi = pown[i];
+                T rv = r[i];
+                if (!fixed) {
+                    x[i] += alpha64 * (double)pi;
+                    rv -= alpha * q[i];
+                    r[i] = rv;
+                }
+                const T zv = fixed ? (T)0 : dinv[i] * rv;
+                P2 g;
+                g.x = zv;
+                g.y = pi;
+                pair[d0 + i] = g;
+                rz += (double)rv * (double)zv;
+                rr += (double)rv * (double)rv;
+            }
+            part[0] = rz;
+            part[1] = rr;
+            ok = rs_sync<2, true>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+        } else if (ph == PH_R && sizeof(T) == 8) {
+            // FP64 true residual from the slices, x in the halo's place
+            double *hx = (double *)halo;
+            const int nh = nu * BS;
+            for (int i0 = tid; i0 < nh; i0 += 4 * RT) {
+                double g[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = i0 + k * RT < nh ? i0 + k * RT : i0;
+                    const int e = BS == 1 ? i : i / 3;
+                    g[k] = __ldcg(S.x + (int64_t)BS * list[e] + (BS == 1 ? 0 : i - 3 * e));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i0 + k * RT < nh) hx[i0 + k * RT] = g[k];
+            }
+            __syncthreads();
+            double rr = 0.0, rp = 0.0, rz = 0.0, aa = 0.0;
+            const int grp = lane >> lsh;
+            const bool first = (lane & (L - 1)) == 0;
+            for (int s = wid; s < nsl; s += RWARPS) {
+                const int off = so[s], w = (so[s + 1] - off) >> 5;
+                const int pos = s * (32 >> lsh) + grp;
+                const int rl = (pos & ~(RS_WINDOW - 1)) + perm[pos];
+                double hi[BS], lo[BS], ab[BS];
+#pragma unroll
+                for (int c = 0; c < BS; ++c) hi[c] = lo[c] = ab[c] = 0.0;
+                if (s < nres)
+                    rs_row_dd<BS, true>(mc + off + lane, (const double *)mv + B2 * (size_t)off + lane, w, hx,
+                                        hi, lo, ab);
+                else
+                    rs_row_dd<BS, false>(gc + off + lane, (const double *)gv + B2 * (size_t)off + lane, w, hx,
+                                         hi, lo, ab);
+                for (int o = L >> 1; o > 0; o >>= 1)
+#pragma unroll
+                    for (int c = 0; c < BS; ++c) {
+                        const double h2 = __shfl_xor_sync(0xffffffffu, hi[c], o);
+                        const double l2 = __shfl_xor_sync(0xffffffffu, lo[c], o);
+                        dd_add(hi[c], lo[c], h2, l2);
+                        ab[c] += __shfl_xor_sync(0xffffffffu, ab[c], o);
+                    }
+                if (rl < nloc && first) {
+#pragma unroll
+                    for (int c = 0; c < BS; ++c) {
+                        const int i = rl * BS + c;
+                        const bool fixed = fx && fx[i];
+                        const double rt = fixed ? 0.0 : dd_residual(__ldg(S.b + d0 + i), hi[c], lo[c]);
+                        rr += rt * rt;
+                        if (!fixed) aa += ab[c] * ab[c];
+                        const T rv = (T)rt;
+                        r[i] = rv;
+                        P2 g = pair[d0 + i];
+                        g.x = fixed ? (T)0 : dinv[i] * rv;
+                        pair[d0 + i] = g;
+                        rz += (double)rv * (double)g.x;
+                        rp += (double)rv * (double)g.y;
+                    }
+                }
+            }
+            part[0] = rr;
+            part[1] = rp;
+            part[2] = rz;
+            part[3] = aa;
+            ok = rs_sync<4, true>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+        } else if (ph == PH_INIT || ph == PH_R) {
+            // FP64 true residual from the FP64 CSR, 8 lanes per row
+            // (compensated sums); INIT also the Jacobi inverse and |b_lift|
+            const bool init = ph == PH_INIT;
+            const int sub = lane & (LANES - 1), grp = lane / LANES;
+            double rr = 0.0, s1 = 0.0, rz = 0.0, aa = 0.0;
+            bool bad = false;
+            for (int base = wid * RPP; base < nloc; base += RWARPS * RPP) {
+                const int rl = base + grp;
+                const bool valid = rl < nloc;
+                const int64_t row = r0 + (valid ? rl : 0);
+                double acc[BS], alo[BS], accf[BS], aab[BS], dg[B2];
+#pragma unroll
+                for (int c = 0; c < BS; ++c) acc[c] = alo[c] = accf[c] = aab[c] = 0.0;
+#pragma unroll
+                for (int c = 0; c < B2; ++c) dg[c] = 0.0;
+                if (valid) {
+                    const int32_t k1 = __ldg(S.rp + row + 1);
+                    if (init)
+                        for (int32_t k = __ldg(S.rp + row) + sub; k < k1; k += LANES)
+                            acc_R<true, BS>(S.v64, S.ci, k, row, S.x, S.fixed, acc, alo, aab, accf, dg);
+                    else
+                        for (int32_t k = __ldg(S.rp + row) + sub; k < k1; k += LANES)
+                            acc_R<false, BS>(S.v64, S.ci, k, row, S.x, S.fixed, acc, alo, aab, accf, dg);
+                }
+#pragma unroll
+                for (int c = 0; c < BS; ++c) {
+                    group_sum_dd<LANES>(acc[c], alo[c]);
+                    aab[c] = group_sum<LANES>(aab[c]);
+                    if (init) {
+                        accf[c] = group_sum<LANES>(accf[c]);
+                        dg[c * BS + c] = group_sum<LANES>(dg[c * BS + c]);
+                    }
+                }
+                if (valid && sub == 0) {
+#pragma unroll
+                    for (int c = 0; c < BS; ++c) {
+                        const int i = rl * BS + c;
+                        const bool fixed = fx && fx[i];
+                        const double bi = __ldg(S.b + d0 + i);
+                        const double rt = fixed ? 0.0 : dd_residual(bi, acc[c], alo[c]);
+                        rr += rt * rt;
+                        if (!fixed) aa += aab[c] * aab[c];
+                        const T rv = (T)rt;
+                        r[i] = rv;
+                        T dv;
+                        if (init) {
+                            double iv = 0.0;
+                            if (!fixed) {
+                                const double d = dg[c * BS + c];
+                                const double bl = bi - accf[c];
+                                s1 += bl * bl;
+                                if (!(d > 0.0) || !isfinite(d)) bad = true;
+                                else iv = 1.0 / d;
+                            }
+                            dv = (T)iv;
+                            dinv[i] = dv;
+                        } else {
+                            dv = dinv[i];
+                        }
+                        const T zv = fixed ? (T)0 : dv * rv;
+                        rz += (double)rv * (double)zv;
+                        P2 g;
+                        g.x = zv;
+                        g.y = init ? (T)0 : pown[i];
+                        if (!init) s1 += (double)rv * (double)g.y;
+                        pair[d0 + i] = g;
+                    }
+                }
+            }
+            part[0] = rr;
+            part[1] = s1;
+            part[2] = rz;
+            part[3] = bad ? -INFINITY : aa;   // a bad diagonal: reported as a breakdown
+            ok = rs_sync<4, true>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+        } else {                              // zero right-hand side
+            for (int i = tid; i < nd; i += RT)
+                if (!(fx && fx[i])) S.x[d0 + i] = 0.0;
+            ok = rs_sync<1, false>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+        }
+        if (!ok) return;
+        ph = sh.st.phase;
+        if (ph == PH_DONE) break;
+    }
+    if (cta == 0 && tid == 0) gst[me.sys] = sh.st;
+}
+
+// ------------------------------------------------------------------ set-up
+// A block's columns as a bitmap over the system's rows in shared memory:
+// marked from the block's rows (and the rows themselves: an absent diagonal
+// still takes slot 0), counted, and ranked by 4-word groups.
+__host__ __device__ inline int rs_words(int64_t n) { return (int)((n + 127) / 128) * 4; }
+
+__device__ __forceinline__ void rs_mark(const SysDev &S, int64_t r0, int nloc, uint32_t *bits,
+                                        int *len) {
+    const int lane = threadIdx.x & 31, sub = lane & 7, wid = threadIdx.x >> 5;
+    for (int base = wid * 4; base < nloc; base += RWARPS * 4) {
+        const int i = base + (lane >> 3);
+        const bool valid = i < nloc;
+        const int64_t row = r0 + i;
+        const int32_t kb = valid ? __ldg(S.rp + row) : 0, ke = valid ? __ldg(S.rp + row + 1) : 0;
+        int diag = 0;
+        for (int32_t k = kb + sub; k < ke; k += 8) {
+            const int32_t c = __ldg(S.ci + k);
+            diag |= c == (int32_t)row;
+            if ((uint32_t)c < (uint32_t)S.n) atomicOr(bits + (c >> 5), 1u << (c & 31));
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) diag |= __shfl_xor_sync(0xffffffffu, diag, o);
+        if (valid && sub == 0) {
+            atomicOr(bits + (row >> 5), 1u << (row & 31));
+            if (len) len[i] = ke - kb + (diag ? 0 : 1);
+        }
+    }
+}
+
+// The blocks' rows: bounds of equal work, a row counting its stored entries
+// and `alpha` more (its share of the update and of the halo). With equal
+// rows instead the blocks that hold a Tet10 mesh's vertex rows (65 entries
+// against 28 on average, and numbered first) had twice the others' work.
+__global__ void k_rs_split(const SysDev *__restrict__ sys, RsCta *ctas, int n, int alpha) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const SysDev &S = sys[ctas[i].sys];
+    const int c = ctas[i].cta;
+    const int64_t total = __ldg(S.rp + S.n) + (int64_t)alpha * S.n;
+    auto bound = [&](int k) {   // first row with k / ncta of the work before it
+        const int64_t want = total * k / S.ncta;
+        int64_t lo = 0, hi = S.n;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (__ldg(S.rp + mid) + alpha * mid < want) lo = mid + 1; else hi = mid;
+        }
+        return (int32_t)lo;
+    };
+    const int32_t r0 = bound(c), r1 = c + 1 == S.ncta ? (int32_t)S.n : bound(c + 1);
+    ctas[i].row0 = r0;
+    ctas[i].rows = r1 - r0;
+    // ceil(rows / RS) slices fit before the next block's first
+    ctas[i].sl0 = S.sl0 + (r0 >> (5 - S.lsh)) + c;
+}
+
+// Row order, slice sizes and halo size of every block: windows of RS_WINDOW
+// rows (the last one shorter) sorted by stored length, longest first, ties
+// in row order; a slice is 32 / L positions, its size 32 x its longest
+// row's slots rounded up to whole steps of L.
+__global__ void __launch_bounds__(RT)
+k_rs_rank(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int64_t *sizes_all,
+          int2 *ucnt) {
+    extern __shared__ __align__(16) uint32_t rs_bits[];
+    __shared__ int total;
+    const RsCta me = ctas[blockIdx.x];
+    const SysDev &S = sys[me.sys];
+    const int nw = rs_words(S.n), t = threadIdx.x, lsh = S.lsh, L = 1 << lsh, rs = 32 >> lsh;
+    const int npos = rs_slices(me.rows, lsh) * rs;   // positions: the rows, then padding
+    int *len = (int *)(rs_bits + nw);
+    for (int i = t; i < nw; i += RT) rs_bits[i] = 0;
+    for (int i = t; i < npos; i += RT) len[i] = 0;
+    if (t == 0) total = 0;
+    __syncthreads();
+    rs_mark(S, me.row0, me.rows, rs_bits, len);
+    __syncthreads();
+    int cnt = 0;
+    for (int i = t; i < nw; i += RT) cnt += __popc(rs_bits[i]);
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    if ((t & 31) == 0) atomicAdd(&total, cnt);
+    uint8_t *perm = (uint8_t *)S.sperm + me.sl0 * 32;
+    for (int i = t; i < npos; i += RT) {
+        const int w0 = i & ~(RS_WINDOW - 1), w1 = min(npos, w0 + RS_WINDOW);
+        const int Li = len[i];
+        int rank = 0;
+        for (int u = w0; u < w1; ++u) rank += (len[u] > Li || (len[u] == Li && u < i)) ? 1 : 0;
+        perm[w0 + rank] = (uint8_t)(i - w0);
+        if (rank % rs == 0) sizes_all[me.sl0 + (w0 + rank) / rs] = 32 * (int64_t)((Li + L - 1) >> lsh);
+    }
+    __syncthreads();
+    if (t == 0) ucnt[blockIdx.x] = make_int2(total, me.rows);
+}
+
+// Slot k of a row of `len` entries with its diagonal at dpos (INT_MAX: none):
+// the entry there, or -1 (padding, or an absent diagonal).
+__device__ __forceinline__ int rs_entry(int k, int len, int dpos) {
+    const int e = k == 0 ? (dpos == INT32_MAX ? -1 : dpos) : (k - 1 < dpos ? k - 1 : k);
+    return e < len ? e : -1;
+}
+__device__ __forceinline__ int rs_dpos(const int32_t *ci, int32_t kb, int len, int32_t row, int u, int L) {
+    int dpos = INT32_MAX;
+    for (int k = u; k < len; k += L)
+        if (__ldg(ci + kb + k) == row) {
+            dpos = k;
+            break;
+        }
+    for (int o = L >> 1; o > 0; o >>= 1) dpos = min(dpos, __shfl_xor_sync(0xffffffffu, dpos, o));
+    return dpos;
+}
+
+// Every block's halo list and the slices' local columns (places in that
+// list). A row repeated in the CSR keeps its repeats as entries.
+__global__ void __launch_bounds__(RT)
+k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int umax,
+          int32_t *__restrict__ ulist, uint16_t *__restrict__ scol) {
+    extern __shared__ __align__(16) uint32_t rs_bits[];
+    __shared__ int wsum[RWARPS];
+    const RsCta me = ctas[blockIdx.x];
+    const SysDev &S = sys[me.sys];
+    const int nw = rs_words(S.n), ng = nw / 4, t = threadIdx.x;
+    const int lane = t & 31, wid = t >> 5;
+    int *pre = (int *)(rs_bits + nw);
+    for (int i = t; i < nw; i += RT) rs_bits[i] = 0;
+    __syncthreads();
+    const int64_t r0 = me.row0;
+    rs_mark(S, r0, me.rows, rs_bits, nullptr);
+    __syncthreads();
+    // exclusive prefix of the groups' counts, one run of groups per thread
+    const int per = (ng + RT - 1) / RT, g0 = min(ng, t * per), g1 = min(ng, g0 + per);
+    int sum = 0;
+    for (int g = g0; g < g1; ++g)
+        for (int j = 0; j < 4; ++j) sum += __popc(rs_bits[4 * g + j]);
+    int inc = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+    }
+    if (lane == 31) wsum[wid] = inc;
+    __syncthreads();
+    int base = inc - sum;
+    for (int k = 0; k < wid; ++k) base += wsum[k];
+    int32_t *list = ulist + (size_t)blockIdx.x * umax;
+    for (int g = g0; g < g1; ++g) {
+        pre[g] = base;
+        for (int j = 0; j < 4; ++j) {
+            uint32_t m = rs_bits[4 * g + j];
+            while (m) {
+                const int b = __ffs(m) - 1;
+                list[base++] = 32 * (4 * g + j) + b;
+                m &= m - 1;
+            }
+        }
+    }
+    __syncthreads();
+    const int lsh = S.lsh, L = 1 << lsh, rs = 32 >> lsh, u = lane & (L - 1);
+    auto place = [&](int32_t c) {
+        if ((uint32_t)c >= (uint32_t)S.n) return (uint16_t)0;   // not a column of this matrix
+        const int w = c >> 5, g = w >> 2;
+        int v = pre[g];
+        for (int j = 4 * g; j < w; ++j) v += __popc(rs_bits[j]);
+        return (uint16_t)(v + __popc(rs_bits[w] & ((1u << (c & 31)) - 1u)));
+    };
+    const uint8_t *perm = S.sperm + me.sl0 * 32;
+    for (int s = wid; s < rs_slices(me.rows, lsh); s += RWARPS) {
+        const int64_t off = __ldg(S.soff + me.sl0 + s);
+        const int w = (int)((__ldg(S.soff + me.sl0 + s + 1) - off) >> 5);
+        if (w == 0) continue;
+        const int pos = s * rs + (lane >> lsh);
+        const int rl = (pos & ~(RS_WINDOW - 1)) + __ldg(perm + pos);
+        const int64_t row = r0 + rl;
+        const bool valid = rl < me.rows;
+        const int32_t kb = valid ? __ldg(S.rp + row) : 0, len = valid ? __ldg(S.rp + row + 1) - kb : 0;
+        const int dpos = rs_dpos(S.ci, kb, len, (int32_t)row, u, L);
+        const uint16_t own = place((int32_t)(valid ? row : r0));
+        for (int k = 0; k < w; ++k) {
+            const int e = rs_entry(k * L + u, len, dpos);
+            scol[off + 32 * k + lane] = e >= 0 ? place(__ldg(S.ci + kb + e)) : own;
+        }
+    }
+}
+
+// The slices' values from the CSR, one warp per slice: the diagonal (0 if
+// the pattern has none) in slot 0, the row's other entries in order, 0 as
+// padding. Run again when the values change.
+template <typename T, int BS>
+__global__ void __launch_bounds__(256)
+k_rs_vals(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, T *__restrict__ sval) {
+    constexpr int B2 = BS * BS;
+    const RsCta me = ctas[blockIdx.x];
+    const SysDev &S = sys[me.sys];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwp = blockDim.x >> 5;
+    const int lsh = S.lsh, L = 1 << lsh, rs = 32 >> lsh, u = lane & (L - 1);
+    const T *v = MatVal<T>::get(S);
+    const int64_t r0 = me.row0;
+    const uint8_t *perm = S.sperm + me.sl0 * 32;
+    for (int s = blockIdx.y * nwp + wid; s < rs_slices(me.rows, lsh); s += gridDim.y * nwp) {
+        const int64_t off = __ldg(S.soff + me.sl0 + s);
+        const int w = (int)((__ldg(S.soff + me.sl0 + s + 1) - off) >> 5);
+        if (w == 0) continue;
+        const int pos = s * rs + (lane >> lsh);
+        const int rl = (pos & ~(RS_WINDOW - 1)) + __ldg(perm + pos);
+        const int64_t row = r0 + rl;
+        const bool valid = rl < me.rows;
+        const int32_t kb = valid ? __ldg(S.rp + row) : 0, len = valid ? __ldg(S.rp + row + 1) - kb : 0;
+        const int dpos = rs_dpos(S.ci, kb, len, (int32_t)row, u, L);
+        for (int k = 0; k < w; ++k) {
+            const int e = rs_entry(k * L + u, len, dpos);
+            T *dst = sval + B2 * (off + 32 * (int64_t)k) + lane;
+#pragma unroll
+            for (int c = 0; c < B2; ++c)
+                dst[32 * c] = e >= 0 ? __ldg(v + ((int64_t)kb + e) * B2 + c) : (T)0;
+        }
+    }
+}

@@ -1,4 +1,7 @@
-// Persistent batched Jacobi-PCG (replaces spla.spsolve / spla.factorized).
+// Batched Jacobi-PCG (replaces spla.spsolve / spla.factorized): phases,
+// schedulers and plans. The resident scheduler, which takes most solves of
+// one or a few systems, is in cfem_resident.cuh; the graph scheduler below
+// takes large batches and solve slots; what neither takes runs as follows.
 //
 // All systems of a batch are solved by ONE cooperative launch (after one
 // ordinary INIT launch). Rows of each system are cut into small chunks
@@ -57,6 +60,7 @@ constexpr double FLOOR_C = 16.0 * 2.220446049250313e-16;
 constexpr double FLOOR_TIGHT = 2.0 * 2.220446049250313e-16;
 constexpr int BAR_GROUP = 16;              // blocks per first-level counter
 constexpr int BAR_MAX_GROUPS = 64;
+constexpr int RS_MAX_CTAS = 160;           // blocks of one resident system, at most
 
 __host__ __device__ inline int chunk_rows(int bs) { return bs == 3 ? 8 : 16; }
 
@@ -110,6 +114,12 @@ struct SysDev {
                           // 0 means 8)
     int32_t rsell;        // bs 1, mixed, A phase staged: an FP64 sliced-ELL copy
                           // (scol / sval / soff / sperm) for the residual phase
+    // resident scheduler: blocks, log2 of the lanes per row, the system's
+    // place in the batch's slice table; (z, p) pairs and the partial sums
+    int32_t ncta, lsh;
+    int64_t sl0;
+    void *pair;
+    ulonglong2 *mail;
 };
 
 struct SysState {
@@ -718,9 +728,11 @@ __device__ __forceinline__ void run_R(const SysDev &S, const SysState *st, int64
         phase_R<T, BS, false, true>(S, st, r0, r1, lane, part, bad);
 }
 
-// State transition of a system once all its chunk sums are in.
+// State transition of a system once all its chunk sums are in. lead: the
+// one caller of a system that also keeps its history and the active count
+// (every block of the resident scheduler advances a state of its own).
 __device__ void advance(const SysDev &S, SysState *st, GridBar *bar, int ph,
-                        const double tot[4]) {
+                        const double tot[4], bool lead = true) {
     const double rtol2 = S.rtol2;
     int next = PH_DONE;
     const int status_now = *(volatile int32_t *)&st->status;
@@ -779,7 +791,7 @@ __device__ void advance(const SysDev &S, SysState *st, GridBar *bar, int ph,
         const double rr = tot[0], rp = tot[1], rz = tot[2], bb = st->bb;
         const double floor2 = FLOOR_TIGHT * FLOOR_TIGHT * tot[3];
         const double loose2 = FLOOR_C * FLOOR_C * tot[3];
-        if (st->nres < S.hist_cap) {
+        if (lead && st->nres < S.hist_cap) {
             S.hist[2 * st->nres] = (double)st->iter;
             S.hist[2 * st->nres + 1] = sqrt(rr / bb);
         }
@@ -818,7 +830,7 @@ __device__ void advance(const SysDev &S, SysState *st, GridBar *bar, int ph,
         next = PH_DONE;
     }
     st->phase = next;
-    if (next == PH_DONE) atomicSub(&bar->active, 1);
+    if (lead && next == PH_DONE) atomicSub(&bar->active, 1);
 }
 
 // Chunk partial -> tile partial -> system total, each level summed in a
@@ -2983,6 +2995,8 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle h, GridBar *bar, unsigned
         cudaGraphSetConditional(h, (act > 0 && r < max_rounds && err == 0) ? 1u : 0u);
     }
 }
+#include "cfem_resident.cuh"
+
 }  // namespace cfem
 
 using namespace cfem;
@@ -3124,6 +3138,15 @@ struct cfem_pcg_plan {
     int n_chunks = 0;
     int max_iter = 1;
     bool persistent = true;
+    bool resident = false;        // k_resident: `waves` launches of whole systems
+    std::vector<int2> waves;      // (first block, blocks) in the block table
+    cfem::RsCta *d_ctas = nullptr;   // block table
+    int rs_ctas = 0, rs_smem = 0, rs_vsm = 0, rs_umax = 0;
+    int2 *rs_ucnt = nullptr;         // every block's halo size and rows
+    int32_t *rs_ulist = nullptr;     // every block's halo
+    char *rs_col = nullptr, *rs_val = nullptr;
+    char *arena = nullptr;           // resident set-up without allocations: memory from here
+    size_t arena_bytes = 0, arena_used = 0;
     int grid = 1;
     unsigned long long bar_timeout_ns = 4000000000ull;   // grid-barrier wait limit
     unsigned bar_hold = 0;                               // phantom arrivals (tests)
@@ -3186,8 +3209,11 @@ namespace cfem {
 
 static size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
+static int rs_copies(cfem_pcg_plan *P, cudaStream_t s);
+
 // (Re)build the working copies of the matrix values on stream s.
 static int plan_copies(cfem_pcg_plan *P, cudaStream_t s, int first = 0, int last = -1) {
+    if (P->resident) return rs_copies(P, s);
     if (last < 0) last = P->n_systems;
     std::vector<PadJob> pad_jobs;
     int64_t pad_rows = 0;
@@ -3413,6 +3439,259 @@ static void plan_free(cfem_pcg_plan *P) {
     delete P;
 }
 
+// ------------------------------------------------- resident scheduler, host
+// Shape of one system from its rows, stored blocks and block size alone (the
+// same alone and in a batch). A block takes at least about 2,560 stored
+// entries (1,024 3x3 blocks): more blocks make the two grid-wide sums of an
+// iteration dearer (16 / 63 / 148 blocks: 4.4 / 5.4 / 6.9 us) than their
+// share of the products saves; a 20^3 P1 box ran 9.0, 7.8 and 9.4 us per
+// iteration on 16, 48 and 148 blocks. Lanes per row: scalar rows one per
+// lane (8 lanes: 2.5 us of products instead of 1.0 on a 44,415-row Tet10
+// box), two where a block has too few rows for its warps; 3x3 block rows 4
+// lanes (20 and more blocks per row, Tet10) or 2 (27 x 15 x 13 Tet10 box in
+// FP32: 26.7 / 21.0 / 18.7 / 21.7 us per iteration for 1 / 2 / 4 / 8).
+static void rs_shape(int64_t n, int64_t nnzb, int bs, int num_sms, int &ncta, int &lsh) {
+    const int64_t per = bs == 3 ? 1024 : 2560;
+    ncta = (int)std::max<int64_t>(1, std::min<int64_t>((nnzb + per - 1) / per, num_sms));
+    if (bs == 3) lsh = nnzb >= 20 * n ? 2 : 1;
+    else lsh = n < 192 * (int64_t)ncta ? 1 : 0;
+}
+
+// Work of a row beside its stored entries (k_rs_split), and with it the
+// most rows a block can get.
+static int rs_alpha(int bs) { return bs == 3 ? 4 : 8; }
+static int64_t rs_most_rows(int64_t n, int64_t nnzb, int bs, int ncta) {
+    return std::min<int64_t>(n, (nnzb / rs_alpha(bs) + n) / ncta + 4);
+}
+static size_t rs_map_bytes(int64_t n, int64_t rows, int lsh) {
+    const size_t bits = (size_t)rs_words(n) * 4;
+    return bits + std::max(((size_t)rows + (32 >> lsh)) * 4, bits / 4);
+}
+
+// Whether the batch may run on the resident scheduler, and its launches:
+// every system of one precision and block size, point Jacobi, the set-up's
+// column bitmap within shared memory, each launch as many whole systems as
+// the SMs hold blocks.
+static bool rs_plan(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t *nnzb) {
+    int used = 0, total = 0;
+    P->waves.clear();
+    const int sms = std::min(P->ctx->num_sms, RS_MAX_CTAS);
+    for (int i = 0; i < P->n_systems; ++i) {
+        const cfem_linsys &L = systems[i];
+        if (L.bs != systems[0].bs || L.mode != systems[0].mode ||
+            (L.bs == 3 && L.precond != CFEM_PRECOND_JACOBI))
+            return false;
+        int ncta, lsh;
+        rs_shape(L.n_rows, nnzb[i], L.bs, sms, ncta, lsh);
+        if (rs_map_bytes(L.n_rows, rs_most_rows(L.n_rows, nnzb[i], L.bs, ncta), lsh) >
+            (size_t)RS_SMEM_MAX)
+            return false;
+        if (P->waves.empty() || used + ncta > sms) {
+            P->waves.push_back(make_int2(total, 0));
+            used = 0;
+            if (P->waves.size() > RS_MAX_WAVES) return false;
+        }
+        used += ncta;
+        total += ncta;
+        P->waves.back().y += ncta;
+    }
+    return true;
+}
+
+template <typename T, int BS>
+static int rs_vals(cfem_pcg_plan *P, cudaStream_t s) {
+    const unsigned gy = (unsigned)std::max(1, std::min(16, P->ctx->num_sms * 8 / P->rs_ctas));
+    (void)cudaGetLastError();
+    k_rs_vals<T, BS><<<dim3((unsigned)P->rs_ctas, gy), 256, 0, s>>>(P->d_sys, P->d_ctas, (T *)P->rs_val);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    CFEM_CUDA(cudaGetLastError());
+    return CFEM_OK;
+}
+
+static int rs_copies(cfem_pcg_plan *P, cudaStream_t s) {
+    const SysDev &S = P->hs[0];
+    if (S.mode == CFEM_SOLVE_MIXED) return S.bs == 3 ? rs_vals<float, 3>(P, s) : rs_vals<float, 1>(P, s);
+    return S.bs == 3 ? rs_vals<double, 3>(P, s) : rs_vals<double, 1>(P, s);
+}
+
+static void *rs_kernel(int bs, int mode) {
+    if (mode == CFEM_SOLVE_MIXED)
+        return bs == 3 ? (void *)k_resident<float, 3> : (void *)k_resident<float, 1>;
+    return bs == 3 ? (void *)k_resident<double, 3> : (void *)k_resident<double, 1>;
+}
+
+// Memory of a resident plan: from the library's pool, or from the plan's
+// arena (*out null when that is full).
+static int rs_alloc(cfem_pcg_plan *P, char **out, size_t bytes, cudaStream_t s) {
+    if (!P->arena) return tmp_alloc(out, bytes, s);
+    const bool fits = P->arena_used + align256(bytes) <= P->arena_bytes;
+    *out = fits ? P->arena + P->arena_used : nullptr;
+    if (fits) P->arena_used += align256(bytes);
+    return CFEM_OK;
+}
+
+// Builds the resident plan, or leaves P->resident false (the caller then
+// takes another scheduler) when a block's halo does not fit shared memory
+// or the plan its arena.
+static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t *nnzb,
+                    cudaStream_t s) {
+    cfem_ctx *ctx = P->ctx;
+    const int sms = std::min(ctx->num_sms, RS_MAX_CTAS), ns = P->n_systems;
+    const int bs = systems[0].bs, mode = systems[0].mode;
+    const size_t ts = mode == CFEM_SOLVE_MIXED ? 4 : 8;
+    P->bar_timeout_ns = 1000ull * (unsigned long long)ctx->barrier_timeout_us;
+    P->bar_hold = (unsigned)ctx->barrier_hold;
+    std::vector<SysDev> &hs = P->hs;
+    std::vector<RsCta> ctas;
+    size_t perm_bytes = 0, map_bytes = 0;
+    int64_t nslices = 0;
+    for (int i = 0; i < ns; ++i) {
+        const cfem_linsys &L = systems[i];
+        SysDev &S = hs[i];
+        S.n = L.n_rows;
+        S.bs = L.bs;
+        S.precond = CFEM_PRECOND_JACOBI;
+        S.mode = L.mode;
+        S.max_iter = L.max_iter;
+        S.rp = L.d_row_ptr;
+        S.ci = L.d_col;
+        S.v64 = L.d_vals64;
+        S.v32 = L.d_vals32;
+        S.b = L.d_b;
+        S.x = L.d_x;
+        S.fixed = L.d_fixed;
+        S.nnzb = nnzb[i];
+        S.rtol2 = L.rtol * L.rtol;
+        const double dl = L.reliable_delta > 0.0 ? L.reliable_delta : RELIABLE_DELTA;
+        S.delta2 = dl * dl;
+        S.max_stall = L.max_stall > 0 ? L.max_stall : MAX_STALL;
+        S.hist_cap = L.d_history ? L.history_cap : 0;
+        S.hist = L.d_history;
+        rs_shape(L.n_rows, nnzb[i], bs, sms, S.ncta, S.lsh);
+        S.sl0 = nslices;
+        nslices += (S.n >> (5 - S.lsh)) + S.ncta + 1;
+        for (int c = 0; c < S.ncta; ++c) ctas.push_back(RsCta{i, c, 0, 0, 0});
+        map_bytes = std::max(map_bytes, rs_map_bytes(S.n, rs_most_rows(S.n, nnzb[i], bs, S.ncta), S.lsh));
+    }
+    perm_bytes = align256((size_t)nslices * 32);
+    P->rs_ctas = (int)ctas.size();
+    const size_t copy = align256(ns * sizeof(SysDev)) + align256(ctas.size() * sizeof(RsCta)) +
+                        perm_bytes + 2 * align256((nslices + 1) * 8) + align256(ctas.size() * 8);
+    CFEM_TRY(rs_alloc(P, &P->ws_copy, copy, s));
+    if (!P->ws_copy) return CFEM_OK;
+    size_t oc = 0;
+    auto take_c = [&](size_t b) { char *p = P->ws_copy + oc; oc += align256(b); return (void *)p; };
+    P->d_sys = (SysDev *)take_c(ns * sizeof(SysDev));
+    P->d_ctas = (RsCta *)take_c(ctas.size() * sizeof(RsCta));
+    int64_t *sizes = (int64_t *)take_c((nslices + 1) * 8);
+    int64_t *soff = (int64_t *)take_c((nslices + 1) * 8);
+    P->rs_ucnt = (int2 *)take_c(ctas.size() * 8);
+    uint8_t *perm = (uint8_t *)take_c((size_t)nslices * 32);
+    for (SysDev &S : hs) {
+        S.soff = soff;
+        S.sperm = perm;
+    }
+    CFEM_CUDA(cudaMemcpyAsync(P->d_sys, hs.data(), ns * sizeof(SysDev), cudaMemcpyHostToDevice, s));
+    CFEM_CUDA(cudaMemcpyAsync(P->d_ctas, ctas.data(), ctas.size() * sizeof(RsCta),
+                              cudaMemcpyHostToDevice, s));
+    CFEM_CUDA(cudaMemsetAsync(sizes, 0, (nslices + 1) * sizeof(int64_t), s));
+    CFEM_LAUNCH(k_rs_split, grid_for(P->rs_ctas, 128), 128, 0, s, P->d_sys, P->d_ctas, P->rs_ctas,
+                rs_alpha(bs));
+    CFEM_CUDA(cudaFuncSetAttribute(k_rs_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
+    CFEM_CUDA(cudaFuncSetAttribute(k_rs_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
+    CFEM_LAUNCH(k_rs_rank, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas, sizes, P->rs_ucnt);
+    size_t scan_bytes = 0;
+    char *scan_tmp = nullptr;
+    CFEM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, sizes, soff, nslices + 1, s));
+    CFEM_TRY(rs_alloc(P, &scan_tmp, scan_bytes, s));
+    if (!scan_tmp) return CFEM_OK;
+    CFEM_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, sizes, soff, nslices + 1, s));
+    if (!P->arena) tmp_free(scan_tmp, s);
+    int64_t total = 0;
+    std::vector<int2> ucnt(ctas.size());
+    CFEM_CUDA(cudaMemcpyAsync(&total, soff + nslices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    CFEM_CUDA(cudaMemcpyAsync(ucnt.data(), P->rs_ucnt, ctas.size() * 8, cudaMemcpyDeviceToHost, s));
+    CFEM_CUDA(cudaStreamSynchronize(s));
+    // shared memory of the largest block: its halo always, its vectors if
+    // every block of the batch has room for them
+    int umax = 0;
+    size_t meta = 0, vec = 0;
+    for (size_t c = 0; c < ctas.size(); ++c) {
+        umax = std::max(umax, ucnt[c].x);
+        meta = std::max(meta, rs_meta_bytes(ucnt[c].y, hs[ctas[c].sys].lsh));
+        vec = std::max(vec, rs_vec_bytes(ucnt[c].y, bs, ts));
+    }
+    size_t fixed = meta + rs_halo_bytes(umax, bs, ts);
+    P->rs_vsm = fixed + vec <= (size_t)RS_SMEM_MAX;
+    if (P->rs_vsm) fixed += vec;
+    size_t state = align256(ns * sizeof(SysState)) + align256(sizeof(GridBar));
+    for (const SysDev &S : hs) {
+        const size_t nd = (size_t)S.n * bs;
+        state += align256(nd * 2 * ts) + align256(rs_mail_bytes(S.ncta)) +
+                 (P->rs_vsm ? 0 : 3 * align256(nd * ts));
+    }
+    const size_t ubytes = align256(ctas.size() * (size_t)umax * 4), cbytes = align256((size_t)total * 2);
+    bool take = umax <= 65535 && fixed <= (size_t)RS_SMEM_MAX;   // else too scattered a pattern
+    if (take) {
+        CFEM_TRY(rs_alloc(P, &P->ws_state, state, s));
+        CFEM_TRY(rs_alloc(P, &P->ws_sdata, ubytes + cbytes + align256((size_t)total * bs * bs * ts), s));
+        take = P->ws_state && P->ws_sdata;
+    }
+    if (!take) {
+        if (!P->arena) tmp_free(P->ws_copy, s);
+        P->ws_copy = P->ws_state = P->ws_sdata = nullptr;
+        hs.assign(ns, SysDev{});
+        return CFEM_OK;
+    }
+    P->resident = true;
+    P->persistent = false;
+    P->rs_umax = umax;
+    size_t os = 0;
+    auto take_s = [&](size_t b) { char *p = P->ws_state + os; os += align256(b); return (void *)p; };
+    P->d_st = (SysState *)take_s(ns * sizeof(SysState));
+    P->d_bar = (GridBar *)take_s(sizeof(GridBar));
+    for (SysDev &S : hs) S.mail = (ulonglong2 *)take_s(rs_mail_bytes(S.ncta));
+    P->state_bytes = os;   // what a solve starts from zero: states and words
+    for (SysDev &S : hs) {
+        const size_t nd = (size_t)S.n * bs;
+        S.pair = take_s(nd * 2 * ts);
+        if (!P->rs_vsm) {
+            S.q = take_s(nd * ts);
+            S.r = take_s(nd * ts);
+            S.dinv = take_s(nd * ts);
+        }
+    }
+    CFEM_CUDA(cudaMemcpyAsync(P->d_sys, hs.data(), ns * sizeof(SysDev), cudaMemcpyHostToDevice, s));
+    P->rs_ulist = (int32_t *)P->ws_sdata;
+    P->rs_col = P->ws_sdata + ubytes;
+    P->rs_val = P->rs_col + cbytes;
+    CFEM_LAUNCH(k_rs_cols, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas, umax,
+                P->rs_ulist, (uint16_t *)P->rs_col);
+    // shared memory: the vectors and, if it fits, the whole matrix with some
+    // room for uneven blocks; the most where systems differ
+    const size_t want = fixed + (size_t)total * (2 + (size_t)bs * bs * ts) / P->rs_ctas * 9 / 8 + 4096;
+    P->rs_smem = ns > 1 ? RS_SMEM_MAX
+                        : (int)std::min<size_t>((want + 1023) & ~(size_t)1023, RS_SMEM_MAX);
+    CFEM_CUDA(cudaFuncSetAttribute(rs_kernel(bs, mode), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   RS_SMEM_MAX));
+    return rs_copies(P, s);
+}
+
+static int rs_run(cfem_pcg_plan *P, cudaStream_t w) {
+    const SysDev &S = P->hs[0];
+    int max_steps = 3 * P->max_iter + 16;
+    for (const int2 &wave : P->waves) {
+        void *args[] = {(void *)&P->d_sys, (void *)&P->d_st, (void *)&P->d_bar, (void *)&P->d_ctas,
+                        (void *)&wave.x, (void *)&P->rs_ucnt, (void *)&P->rs_ulist, (void *)&P->rs_umax,
+                        (void *)&P->rs_col, (void *)&P->rs_val, (void *)&P->rs_smem,
+                        (void *)&P->rs_vsm, (void *)&max_steps, (void *)&P->bar_timeout_ns, (void *)&P->bar_hold};
+        CFEM_CUDA(cudaLaunchCooperativeKernel(rs_kernel(S.bs, S.mode), dim3((unsigned)wave.y),
+                                              dim3(RT), args, (size_t)P->rs_smem, w));
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+    }
+    return CFEM_OK;
+}
+
 static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,
                       cudaStream_t s, cfem_pcg_plan *P) {
     P->ctx = ctx;
@@ -3453,6 +3732,14 @@ static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,
                                   cudaMemcpyDeviceToHost, s));
     }
     CFEM_CUDA(cudaStreamSynchronize(s));
+    for (int i = 0; i < n_systems; ++i) max_iter = std::max(max_iter, (int)systems[i].max_iter);
+    P->max_iter = max_iter;
+    if (!P->slots &&
+        (ctx->scheduler == CFEM_SCHED_AUTO || ctx->scheduler == CFEM_SCHED_PERSISTENT) &&
+        rs_plan(P, systems, nnzbs.data())) {
+        CFEM_TRY(rs_build(P, systems, nnzbs.data(), s));
+        if (P->resident) return CFEM_OK;
+    }
     size_t state_bytes = 0, copy_bytes = 0;
     for (int i = 0; i < n_systems; ++i) {
         const cfem_linsys &L = systems[i];
@@ -3491,11 +3778,9 @@ static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,
                        align256(S.ntiles * sizeof(unsigned)) +
                        align256(S.nchunksB * 4 * sizeof(double));
         n_chunks_b += S.nchunksB;
-        if (L.max_iter > max_iter) max_iter = L.max_iter;
     }
     const int n_chunks = (int)chunk_sys.size();
     P->n_chunks = n_chunks;
-    P->max_iter = max_iter;
     int per_sm = 0;
     CFEM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
         &per_sm, k_pcg_persistent, SOLVE_THREADS, 0));
@@ -3837,7 +4122,11 @@ static int plan_run(cfem_pcg_plan *P, cfem_solve_stats *stats, cudaStream_t s) {
     // The plan's stream runs after everything queued so far on s.
     CFEM_CUDA(cudaEventRecord(P->ev[0], s));
     CFEM_CUDA(cudaStreamWaitEvent(w, P->ev[0], 0));
-    if (P->persistent || P->polled) {
+    if (P->resident) {
+        CFEM_CUDA(cudaMemsetAsync(P->ws_state, 0, P->state_bytes, w));
+        CFEM_CUDA(cudaEventRecord(P->ev[2], w));
+        CFEM_TRY(rs_run(P, w));
+    } else if (P->persistent || P->polled) {
         CFEM_CUDA(cudaMemsetAsync(P->ws_state, 0, P->state_bytes, w));
         P->h_flags[2] = n_systems;
         CFEM_CUDA(cudaMemcpyAsync(&d_bar->active, &P->h_flags[2], sizeof(int),
@@ -3846,7 +4135,9 @@ static int plan_run(cfem_pcg_plan *P, cfem_solve_stats *stats, cudaStream_t s) {
         CFEM_LAUNCH(k_pcg_init, grid_for((int64_t)n_chunks * 32, 256), 256, 0, w,
                     d_sys, d_st, P->d_chunks, n_chunks, d_bar);
     }
-    if (P->persistent) {
+    if (P->resident) {
+        // queued above
+    } else if (P->persistent) {
         void *args[] = {(void *)&d_sys, (void *)&d_st, (void *)&P->d_chunks,
                         (void *)&n_chunks, (void *)&d_bar, (void *)&max_steps,
                         (void *)&P->bar_timeout_ns, (void *)&P->bar_hold};
@@ -3887,7 +4178,7 @@ static int plan_run(cfem_pcg_plan *P, cfem_solve_stats *stats, cudaStream_t s) {
     }
     CFEM_CUDA(cudaEventRecord(P->ev[3], w));
     // states, error word and loop rounds into pinned memory: one wait
-    const bool graph_loop = !P->persistent && !P->polled;
+    const bool graph_loop = !P->persistent && !P->polled && !P->resident;
     CFEM_CUDA(cudaMemcpyAsync(P->h_st, d_st, n_systems * sizeof(SysState),
                               cudaMemcpyDeviceToHost, w));
     CFEM_CUDA(cudaMemcpyAsync(&P->h_flags[3], &d_bar->err, sizeof(int),
@@ -4362,6 +4653,32 @@ static int noalloc_scratch(void **out) {
 
 }  // namespace cfem
 
+// Reads the outcome of a solve on the fixed array into *stats.
+static int noalloc_result(const cfem::SysState *d_st, const cfem::GridBar *d_bar,
+                          cfem_solve_stats *stats, cudaStream_t s) {
+    SysState hst;
+    int h_err = 0;
+    CFEM_CUDA(cudaMemcpyAsync(&hst, d_st, sizeof(SysState), cudaMemcpyDeviceToHost, s));
+    CFEM_CUDA(cudaMemcpyAsync(&h_err, &d_bar->err, sizeof(int),
+                              cudaMemcpyDeviceToHost, s));
+    CFEM_CUDA(cudaStreamSynchronize(s));
+    stats->status = hst.status;
+    if (hst.status == CFEM_OK && hst.phase != PH_DONE)
+        stats->status = CFEM_ERR_NOT_CONVERGED;
+    stats->iterations = hst.iter;
+    stats->residual_updates = hst.nres;
+    stats->pad_ = 0;
+    stats->relres = hst.relres;
+    stats->bnorm = sqrt(hst.bb);
+    stats->kernel_ms = 0.0;
+    stats->spmv_ms = 0.0;
+    stats->spmv_samples = 0;
+    stats->pad2_ = 0;
+    CFEM_CHECK(h_err == 0, CFEM_ERR_TIMEOUT,
+               "solver grid barrier timed out (device wait bound reached)");
+    return CFEM_OK;
+}
+
 extern "C" size_t cfem_pcg_noalloc_capacity(void) { return NOALLOC_SCRATCH_BYTES; }
 
 extern "C" int cfem_pcg_solve_noalloc(cfem_ctx *ctx, const cfem_linsys *L,
@@ -4427,6 +4744,27 @@ extern "C" int cfem_pcg_solve_noalloc(cfem_ctx *ctx, const cfem_linsys *L,
     void *base = nullptr;
     CFEM_TRY(noalloc_scratch(&base));
     char *ws = (char *)base;
+    // the resident scheduler, when its working set fits the array too (the
+    // same choice and arithmetic as cfem_pcg_solve then)
+    {
+        int32_t nnzb = 0;
+        CFEM_CUDA(cudaMemcpyAsync(&nnzb, L->d_row_ptr + L->n_rows, sizeof(int32_t),
+                                  cudaMemcpyDeviceToHost, s));
+        CFEM_CUDA(cudaStreamSynchronize(s));
+        cfem_pcg_plan P;
+        P.ctx = ctx;
+        P.n_systems = 1;
+        P.max_iter = L->max_iter;
+        P.hs.assign(1, SysDev{});
+        P.arena = ws;
+        P.arena_bytes = NOALLOC_SCRATCH_BYTES;
+        if (rs_plan(&P, L, &nnzb)) CFEM_TRY(rs_build(&P, L, &nnzb, s));
+        if (P.resident) {
+            CFEM_CUDA(cudaMemsetAsync(P.ws_state, 0, P.state_bytes, s));
+            CFEM_TRY(rs_run(&P, s));
+            return noalloc_result(P.d_st, P.d_bar, stats, s);
+        }
+    }
     // Every call reuses the array: clear all of it that this call uses
     // (state, tickets, chunk table, p buffers) before the launch.
     CFEM_CUDA(cudaMemsetAsync(ws, 0, need, s));
@@ -4470,26 +4808,6 @@ extern "C" int cfem_pcg_solve_noalloc(cfem_ctx *ctx, const cfem_linsys *L,
     CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_pcg_persistent, dim3(grid),
                                           dim3(SOLVE_THREADS), args, 0, s));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    SysState hst;
-    int h_err = 0;
-    CFEM_CUDA(cudaMemcpyAsync(&hst, d_st, sizeof(SysState), cudaMemcpyDeviceToHost, s));
-    CFEM_CUDA(cudaMemcpyAsync(&h_err, &d_bar->err, sizeof(int),
-                              cudaMemcpyDeviceToHost, s));
-    CFEM_CUDA(cudaStreamSynchronize(s));
-    stats->status = hst.status;
-    if (hst.status == CFEM_OK && hst.phase != PH_DONE)
-        stats->status = CFEM_ERR_NOT_CONVERGED;
-    stats->iterations = hst.iter;
-    stats->residual_updates = hst.nres;
-    stats->pad_ = 0;
-    stats->relres = hst.relres;
-    stats->bnorm = sqrt(hst.bb);
-    stats->kernel_ms = 0.0;
-    stats->spmv_ms = 0.0;
-    stats->spmv_samples = 0;
-    stats->pad2_ = 0;
-    CFEM_CHECK(h_err == 0, CFEM_ERR_TIMEOUT,
-               "solver grid barrier timed out (device wait bound reached)");
-    return CFEM_OK;
+    return noalloc_result(d_st, d_bar, stats, s);
     CFEM_API_END
 }

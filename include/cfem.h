@@ -141,8 +141,14 @@ CFEM_API int cfem_version(void);
 CFEM_API int cfem_ctx_create(int device, cfem_ctx **out);
 CFEM_API int cfem_ctx_destroy(cfem_ctx *ctx);
 /* How cfem_pcg_solve runs its iterations:
- * PERSISTENT    - one cooperative launch, grid barrier between phases
- *                 (lowest latency when the whole batch fits in one wave);
+ * PERSISTENT    - cooperative launches that keep the whole solve on the
+ *                 device, the grid meeting between the phases. Systems of
+ *                 one precision and block size with point Jacobi run on the
+ *                 resident kernel (vectors, matrix slices and the direction's
+ *                 halo in shared memory, the rest of the matrix streamed);
+ *                 others (3x3 block Jacobi, mixed kinds, patterns too
+ *                 scattered or systems too large for the halo) on one launch
+ *                 over the CSR arrays;
  * GRAPH         - per-phase kernels with a warp per row chunk (direction,
  *                 SpMV, reduction, update, reduction per iteration); the
  *                 whole solve is ONE CUDA graph launch whose device-side
@@ -151,8 +157,9 @@ CFEM_API int cfem_ctx_destroy(cfem_ctx *ctx);
  * GRAPH_POLLED  - the same kernels replayed from plain graphs of 16
  *                 iterations, the host polling convergence once per replay
  *                 (every launch visible to per-launch profilers);
- * AUTO          - PERSISTENT when all row chunks fit in one resident wave,
- *                 else GRAPH (default). */
+ * AUTO          - the resident kernel where it takes the systems in at most
+ *                 four launches; else PERSISTENT when all row chunks fit in
+ *                 one resident wave, else GRAPH (default). */
 enum { CFEM_SCHED_AUTO = 0, CFEM_SCHED_PERSISTENT = 1, CFEM_SCHED_GRAPH = 2,
        CFEM_SCHED_GRAPH_POLLED = 3 };
 CFEM_API int cfem_ctx_set_scheduler(cfem_ctx *ctx, int scheduler);
@@ -442,11 +449,11 @@ CFEM_API int cfem_mixed_matrix_batch(cfem_ctx *ctx, const cfem_mixed_job *jobs,
                                      int32_t n_jobs, void *stream);
 
 /* ---- solver -------------------------------------------------------------
- * Jacobi-preconditioned CG on a batch of independent systems. Batches whose
- * work fits one resident wave run in ONE persistent cooperative launch (two
- * grid barriers per iteration); larger ones replay captured CUDA graphs of
- * 16 iterations (direction update, SpMV, reduction, update, reduction per
- * iteration). Per-system scalars are reduced in a fixed order, so each
+ * Jacobi-preconditioned CG on a batch of independent systems. A few systems
+ * of one kind run on the resident kernel (whole solves in cooperative
+ * launches, two grid-wide sums per iteration); larger batches are one graph
+ * of per-phase launches (direction update, SpMV, reduction, update,
+ * reduction per iteration). Per-system scalars are reduced in a fixed order, so each
  * result is bitwise the same alone and in any batch on a given scheduler.
  * CFEM_SOLVE_MIXED runs the CG in FP32 and keeps FP64 for the true residual
  * r = b - A x, the solution update and the convergence test (reliable
@@ -539,12 +546,15 @@ CFEM_API int cfem_cocg_solve(cfem_ctx *ctx, int64_t n, const int32_t *d_indptr,
  * not reset the device (cudaDeviceReset) after it. Every call reuses the
  * same array and clears it first: calls that overlap on the GPU (other
  * streams, other threads) race and must be serialised by the caller.
- * It always runs the persistent scheduler (one cooperative launch, the
- * grid strided over the row chunks when they exceed one resident wave):
- * the context's scheduler, SpMV staging and tuned solve-loop parameters have
- * no effect (its grid-barrier wait limit does), and stats->kernel_ms and
+ * It always runs the persistent scheduler (the resident kernel when its
+ * working set, about 12 bytes per FP64 entry of a scalar matrix and 3 vectors,
+ * fits the array, else one cooperative launch over the CSR arrays, the grid
+ * strided over the row chunks when they exceed one resident wave): the
+ * context's scheduler, SpMV staging and tuned solve-loop parameters have no
+ * effect (its grid-barrier wait limit does), and stats->kernel_ms and
  * stats->spmv_ms are 0 (no timing events are created). The arithmetic is
- * that of cfem_pcg_solve on the persistent scheduler. Synchronises. */
+ * that of cfem_pcg_solve on the persistent scheduler, where the array holds
+ * the resident kernel's working set. Synchronises. */
 CFEM_API size_t cfem_pcg_noalloc_capacity(void);
 CFEM_API int cfem_pcg_solve_noalloc(cfem_ctx *ctx, const cfem_linsys *system,
                                     cfem_solve_stats *stats, void *stream);
