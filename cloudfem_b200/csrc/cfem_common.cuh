@@ -142,6 +142,11 @@ inline unsigned grid_for(int64_t n, int block) {
 
 int set_device(int device);
 
+// COCG in one cooperative launch (cfem_solve.cu); *taken: whether it ran.
+int cocg_resident(cfem_ctx *ctx, int64_t n, const int32_t *ip, const int32_t *ix, const double *vals,
+                  const double *b, double *x, double rtol, int max_iter, cfem_solve_stats *stats,
+                  cudaStream_t s, bool *taken);
+
 // ---------------------------------------------------------------- device
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll

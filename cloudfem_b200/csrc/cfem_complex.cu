@@ -3,6 +3,8 @@
 // eddy-current system of em3d_tet10.py:267-375 once its V rows are scaled
 // by 1/(i omega), which makes the system complex symmetric (A^T = A).
 //
+// Most systems run in one cooperative launch (cfem_cocg.cuh); this file has
+// the interface and the general path, for patterns too scattered for it.
 // Complex values are interleaved (re, im) doubles. Every iteration is five
 // launches (SpMV + p.q, alpha, update + r.z and |r|^2, beta and the
 // convergence test, direction); block partial sums are reduced in block
@@ -271,6 +273,10 @@ extern "C" int cfem_cocg_solve(cfem_ctx *ctx, int64_t n, const int32_t *d_indptr
                CFEM_ERR_INVALID, "complex arrays must be 16-byte aligned");
     CFEM_TRY(set_device(ctx->device));
     cudaStream_t s = (cudaStream_t)stream;
+    bool taken = false;
+    CFEM_TRY(cocg_resident(ctx, n, d_indptr, d_indices, d_vals, d_b, d_x, rtol, max_iter, stats, s,
+                           &taken));
+    if (taken) return CFEM_OK;
     const unsigned nb_rows = grid_for(n, CW);                 // warp per row
     unsigned nb_vec = grid_for(n, CT);
     if (nb_vec > (unsigned)ctx->num_sms * 8) nb_vec = ctx->num_sms * 8;

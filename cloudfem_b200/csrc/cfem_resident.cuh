@@ -113,16 +113,16 @@ __device__ __forceinline__ bool mail_get(const ulonglong2 *p, unsigned long long
 }
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
-// Grid-wide sum of NV quantities over the system's blocks, then the state
-// transition, in every block for itself. PUB: what the block wrote to
-// global memory before is visible to the system's other blocks after it,
-// and theirs to this one (the product phase writes nothing others read and
-// goes without). Returns false when a block gave up waiting (bounded:
-// timeout_ns).
-template <int NV, bool PUB>
-__device__ __forceinline__ bool rs_sync(const SysDev &S, RsShared &sh, GridBar *bar, int cta,
-                                        int ph, unsigned long long epoch, double part[4],
-                                        unsigned long long timeout_ns, unsigned hold) {
+// Grid-wide sum of NV quantities over a system's blocks, then the state
+// transition adv(totals), in every block for itself (one thread). PUB: what
+// the block wrote to global memory before is visible to the system's other
+// blocks after it, and theirs to this one (the product phase writes nothing
+// others read and goes without). Returns false when a block gave up waiting
+// (bounded: timeout_ns).
+template <int NV, bool PUB, typename Shared, typename Adv>
+__device__ __forceinline__ bool rs_sync(Shared &sh, ulonglong2 *mail, int nc, GridBar *bar, int cta,
+                                        unsigned long long epoch, double part[4],
+                                        unsigned long long timeout_ns, unsigned hold, Adv adv) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int v = 0; v < NV; ++v) part[v] = warp_sum(part[v]);
@@ -140,11 +140,11 @@ __device__ __forceinline__ bool rs_sync(const SysDev &S, RsShared &sh, GridBar *
             tot[v] = t;
         }
         bool ok = true;
-        if (S.ncta > 1 || hold) {
-            const int nc = S.ncta, R = rs_copies_of(nc);
+        if (nc > 1 || hold) {
+            const int R = rs_copies_of(nc);
             // two sets of words in turn: a block writes set e + 2 only after
             // every block has written, and so read past, set e
-            ulonglong2 *box = S.mail + (size_t)(epoch & 1) * 4 * R * nc;
+            ulonglong2 *box = mail + (size_t)(epoch & 1) * 4 * R * nc;
             if (PUB) fence_gpu();    // the block's writes before its words
             if (lane < R)
 #pragma unroll
@@ -190,12 +190,8 @@ __device__ __forceinline__ bool rs_sync(const SysDev &S, RsShared &sh, GridBar *
                 }
         }
         if (lane == 0) {
-            if (!ok) {
-                sh.quit = 1;
-            } else {
-                if (ph == PH_INIT && tot[3] < 0.0) sh.st.status = CFEM_ERR_BREAKDOWN;
-                advance(S, &sh.st, bar, ph, tot, cta == 0);
-            }
+            if (ok) adv(tot);
+            else sh.quit = 1;
         }
     }
     __syncthreads();
@@ -422,6 +418,10 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
 
     int ph = PH_INIT;
     unsigned long long epoch = 0;
+    auto adv = [&](const double tot[4]) {
+        if (ph == PH_INIT && tot[3] < 0.0) sh.st.status = CFEM_ERR_BREAKDOWN;
+        advance(S, &sh.st, bar, ph, tot, cta == 0);
+    };
     for (int step = 0; step < max_steps; ++step) {
         double part[4] = {0.0, 0.0, 0.0, 0.0};
         ++epoch;
@@ -482,7 +482,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                 }
             }
             part[0] = pq;
-            ok = rs_sync<1, false>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+            ok = rs_sync<1, false>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
         } else if (ph == PH_B) {
             const double alpha64 = sh.st.alpha;
             const T alpha = (T)alpha64;
@@ -507,7 +507,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
             }
             part[0] = rz;
             part[1] = rr;
-            ok = rs_sync<2, true>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+            ok = rs_sync<2, true>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
         } else if (ph == PH_R && sizeof(T) == 8) {
             // FP64 true residual from the slices, x in the halo's place
             double *hx = (double *)halo;
@@ -571,7 +571,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
             part[1] = rp;
             part[2] = rz;
             part[3] = aa;
-            ok = rs_sync<4, true>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+            ok = rs_sync<4, true>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
         } else if (ph == PH_INIT || ph == PH_R) {
             // FP64 true residual from the FP64 CSR, 8 lanes per row
             // (compensated sums); INIT also the Jacobi inverse and |b_lift|
@@ -646,11 +646,11 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
             part[1] = s1;
             part[2] = rz;
             part[3] = bad ? -INFINITY : aa;   // a bad diagonal: reported as a breakdown
-            ok = rs_sync<4, true>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+            ok = rs_sync<4, true>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
         } else {                              // zero right-hand side
             for (int i = tid; i < nd; i += RT)
                 if (!(fx && fx[i])) S.x[d0 + i] = 0.0;
-            ok = rs_sync<1, false>(S, sh, bar, cta, ph, epoch, part, timeout_ns, hold);
+            ok = rs_sync<1, false>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
         }
         if (!ok) return;
         ph = sh.st.phase;
@@ -868,7 +868,7 @@ k_rs_vals(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, T *__r
             T *dst = sval + B2 * (off + 32 * (int64_t)k) + lane;
 #pragma unroll
             for (int c = 0; c < B2; ++c)
-                dst[32 * c] = e >= 0 ? __ldg(v + ((int64_t)kb + e) * B2 + c) : (T)0;
+                dst[32 * c] = e >= 0 ? __ldg(v + ((int64_t)kb + e) * B2 + c) : T{};
         }
     }
 }

@@ -242,6 +242,9 @@ template <> struct MatVal<double> {
 template <> struct MatVal<float> {
     static __device__ __forceinline__ const float *get(const SysDev &S) { return S.v32; }
 };
+template <> struct MatVal<double2> {   // complex systems: interleaved values
+    static __device__ __forceinline__ const double2 *get(const SysDev &S) { return (const double2 *)S.v64; }
+};
 
 // Inverse of the free part of a 3x3 block (fixed rows/cols -> 0).
 __device__ __forceinline__ bool block_inverse(const double a[9], const bool fx[3],
@@ -2996,6 +2999,7 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle h, GridBar *bar, unsigned
     }
 }
 #include "cfem_resident.cuh"
+#include "cfem_cocg.cuh"
 
 }  // namespace cfem
 
@@ -3141,6 +3145,7 @@ struct cfem_pcg_plan {
     bool resident = false;        // k_resident: `waves` launches of whole systems
     std::vector<int2> waves;      // (first block, blocks) in the block table
     cfem::RsCta *d_ctas = nullptr;   // block table
+    size_t rs_ts = 8;                // bytes of a vector entry (complex: 16)
     int rs_ctas = 0, rs_smem = 0, rs_vsm = 0, rs_umax = 0;
     int2 *rs_ucnt = nullptr;         // every block's halo size and rows
     int32_t *rs_ulist = nullptr;     // every block's halo
@@ -3447,14 +3452,19 @@ static void plan_free(cfem_pcg_plan *P) {
 // share of the products saves; a 20^3 P1 box ran 9.0, 7.8 and 9.4 us per
 // iteration on 16, 48 and 148 blocks. Lanes per row: scalar rows one per
 // lane (8 lanes: 2.5 us of products instead of 1.0 on a 44,415-row Tet10
-// box), two where a block has too few rows for its warps; 3x3 block rows 4
-// lanes (20 and more blocks per row, Tet10) or 2 (27 x 15 x 13 Tet10 box in
+// box), more where a block has too few rows for its warps and the rows are
+// long (the phasor system's 90 entries); 3x3 block rows 4 lanes (20 and more blocks per row, Tet10) or 2 (27 x 15 x 13 Tet10 box in
 // FP32: 26.7 / 21.0 / 18.7 / 21.7 us per iteration for 1 / 2 / 4 / 8).
 static void rs_shape(int64_t n, int64_t nnzb, int bs, int num_sms, int &ncta, int &lsh) {
     const int64_t per = bs == 3 ? 1024 : 2560;
     ncta = (int)std::max<int64_t>(1, std::min<int64_t>((nnzb + per - 1) / per, num_sms));
-    if (bs == 3) lsh = nnzb >= 20 * n ? 2 : 1;
-    else lsh = n < 192 * (int64_t)ncta ? 1 : 0;
+    const int64_t mean = nnzb / n, rows = n / ncta;
+    if (bs == 3) {
+        lsh = mean >= 20 ? 2 : 1;
+    } else {
+        lsh = 0;
+        while (lsh < 3 && ((rows << lsh) >> 5) < 12 && (mean >> lsh) >= 16) ++lsh;
+    }
 }
 
 // Work of a row beside its stored entries (k_rs_split), and with it the
@@ -3510,6 +3520,7 @@ static int rs_vals(cfem_pcg_plan *P, cudaStream_t s) {
 
 static int rs_copies(cfem_pcg_plan *P, cudaStream_t s) {
     const SysDev &S = P->hs[0];
+    if (P->rs_ts == 16) return rs_vals<double2, 1>(P, s);
     if (S.mode == CFEM_SOLVE_MIXED) return S.bs == 3 ? rs_vals<float, 3>(P, s) : rs_vals<float, 1>(P, s);
     return S.bs == 3 ? rs_vals<double, 3>(P, s) : rs_vals<double, 1>(P, s);
 }
@@ -3538,7 +3549,8 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     cfem_ctx *ctx = P->ctx;
     const int sms = std::min(ctx->num_sms, RS_MAX_CTAS), ns = P->n_systems;
     const int bs = systems[0].bs, mode = systems[0].mode;
-    const size_t ts = mode == CFEM_SOLVE_MIXED ? 4 : 8;
+    if (mode == CFEM_SOLVE_MIXED) P->rs_ts = 4;
+    const size_t ts = P->rs_ts;
     P->bar_timeout_ns = 1000ull * (unsigned long long)ctx->barrier_timeout_us;
     P->bar_hold = (unsigned)ctx->barrier_hold;
     std::vector<SysDev> &hs = P->hs;
@@ -3672,8 +3684,8 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     const size_t want = fixed + (size_t)total * (2 + (size_t)bs * bs * ts) / P->rs_ctas * 9 / 8 + 4096;
     P->rs_smem = ns > 1 ? RS_SMEM_MAX
                         : (int)std::min<size_t>((want + 1023) & ~(size_t)1023, RS_SMEM_MAX);
-    CFEM_CUDA(cudaFuncSetAttribute(rs_kernel(bs, mode), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   RS_SMEM_MAX));
+    CFEM_CUDA(cudaFuncSetAttribute(ts == 16 ? (void *)k_resident_cocg : rs_kernel(bs, mode),
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
     return rs_copies(P, s);
 }
 
@@ -3690,6 +3702,79 @@ static int rs_run(cfem_pcg_plan *P, cudaStream_t w) {
         g_launches.fetch_add(1, std::memory_order_relaxed);
     }
     return CFEM_OK;
+}
+
+// COCG of one complex symmetric system on the resident layout (see
+// cfem_cocg_solve); *taken false, and nothing done, when the layout does not
+// fit.
+int cocg_resident(cfem_ctx *ctx, int64_t n, const int32_t *ip, const int32_t *ix, const double *vals,
+                  const double *b, double *x, double rtol, int max_iter, cfem_solve_stats *stats,
+                  cudaStream_t s, bool *taken) {
+    *taken = false;
+    if (n >= (int64_t)1 << 27) return CFEM_OK;
+    int32_t nnz = 0;
+    CFEM_CUDA(cudaMemcpyAsync(&nnz, ip + n, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    CFEM_CUDA(cudaStreamSynchronize(s));
+    cfem_linsys L;
+    memset(&L, 0, sizeof(L));
+    L.n_rows = n;
+    L.bs = 1;
+    L.d_row_ptr = ip;
+    L.d_col = ix;
+    L.d_vals64 = vals;
+    L.d_b = b;
+    L.d_x = x;
+    L.rtol = rtol;
+    L.max_iter = max_iter;
+    cfem_pcg_plan P;
+    P.ctx = ctx;
+    P.n_systems = 1;
+    P.max_iter = max_iter;
+    P.rs_ts = 16;
+    P.hs.assign(1, SysDev{});
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    int st = CFEM_OK;
+    if (nnz > 0 && rs_plan(&P, &L, &nnz)) st = rs_build(&P, &L, &nnz, s);
+    auto run = [&]() -> int {
+        CFEM_CUDA(cudaEventCreate(&e0));
+        CFEM_CUDA(cudaEventCreate(&e1));
+        CFEM_CUDA(cudaMemsetAsync(P.ws_state, 0, P.state_bytes, s));
+        static_assert(sizeof(CocgState) <= sizeof(SysState), "the state record holds either");
+        CocgState *d_st = (CocgState *)P.d_st;
+        double rtol2 = rtol * rtol;
+        void *args[] = {(void *)&P.d_sys, (void *)&d_st, (void *)&P.d_bar, (void *)&P.d_ctas,
+                        (void *)&P.rs_ucnt, (void *)&P.rs_ulist, (void *)&P.rs_umax,
+                        (void *)&P.rs_col, (void *)&P.rs_val, (void *)&P.rs_smem,
+                        (void *)&P.rs_vsm, (void *)&rtol2, (void *)&max_iter,
+                        (void *)&P.bar_timeout_ns};
+        CFEM_CUDA(cudaEventRecord(e0, s));
+        CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_resident_cocg, dim3((unsigned)P.rs_ctas),
+                                              dim3(RT), args, (size_t)P.rs_smem, s));
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        CFEM_CUDA(cudaEventRecord(e1, s));
+        CocgState h;
+        int err = 0;
+        CFEM_CUDA(cudaMemcpyAsync(&h, d_st, sizeof(h), cudaMemcpyDeviceToHost, s));
+        CFEM_CUDA(cudaMemcpyAsync(&err, &P.d_bar->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CFEM_CUDA(cudaStreamSynchronize(s));
+        float ms = 0.0f;
+        CFEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+        CFEM_CHECK(err == 0, CFEM_ERR_TIMEOUT,
+                   "solver grid barrier timed out (device wait bound reached)");
+        memset(stats, 0, sizeof(*stats));
+        stats->status = h.status;
+        stats->iterations = h.iter;
+        stats->relres = h.bb > 0.0 ? sqrt(h.rr / h.bb) : 0.0;
+        stats->bnorm = sqrt(h.bb);
+        stats->kernel_ms = ms;
+        *taken = true;
+        return CFEM_OK;
+    };
+    if (st == CFEM_OK && P.resident) st = run();
+    if (e0) cudaEventDestroy(e0);
+    if (e1) cudaEventDestroy(e1);
+    for (char *m : {P.ws_copy, P.ws_state, P.ws_sdata}) tmp_free(m, s);
+    return st;
 }
 
 static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,

@@ -175,3 +175,34 @@ def test_zero_load_and_missing_mask(torch):
     s.row_ptr, s.col, s.vals64 = up(A.indptr, np.int32), up(A.indices, np.int32), up(A.data, np.float64)
     s.b.fill_(1.0)
     assert pcg([s], N.SOLVE_FP64, 1e-12, 2000)[0].status == N.CFEM_ERR_BREAKDOWN
+
+
+@pytest.mark.parametrize("n,kind", [(1, "band"), (33, "band"), (700, "arrow"), (9000, "band"),
+                                    (4000, "scatter"), (120000, "band")])
+def test_cocg_matches_direct(torch, n, kind):
+    """Complex symmetric systems (the phasor solver): one block, several, rows
+    longer than a window, entries past shared memory, and a long arrow row.
+    The real part has eigenvalues in [0.2, 2.8] and the imaginary part is a
+    positive diagonal, so a relative residual of 1e-12 bounds the error by
+    about 14e-12 of the solution: 1e-10."""
+    import ctypes
+    from cloudfem_b200 import _native as N
+    rt = N.runtime()
+    A, *_ = _system(n, 1, kind, 7 * n + 1)
+    rng = np.random.default_rng(n)
+    A = (A + 1j * sp.diags(rng.uniform(0.1, 1.0, n))).tocsr()
+    A.sort_indices()
+    b = rng.uniform(-1.0, 1.0, n) + 1j * rng.uniform(-1.0, 1.0, n)
+    up = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(rt.device)  # noqa: E731
+    ip, ix = up(A.indptr.astype(np.int32)), up(A.indices.astype(np.int32))
+    va, vb = up(A.data.view(np.float64)), up(b.view(np.float64))
+    x = torch.zeros(2 * n, dtype=torch.float64, device=rt.device)
+    st = N.SolveStats()
+    N.check(rt.lib.cfem_cocg_solve(rt.ctx, n, N.ptr(ip), N.ptr(ix), N.ptr(va), N.ptr(vb), N.ptr(x),
+                                   1e-12, 2000, ctypes.byref(st), rt.stream()))
+    assert st.status == N.CFEM_OK and st.relres <= 1e-12
+    xs = x.cpu().numpy().view(np.complex128)
+    assert np.linalg.norm(A @ xs - b) <= 2e-12 * np.linalg.norm(b)
+    if kind != "scatter":
+        ref = spla.spsolve(A.tocsc(), b)
+        assert np.linalg.norm(xs - ref) <= 1e-10 * np.linalg.norm(ref)
