@@ -63,9 +63,7 @@ __device__ __forceinline__ double2 cocg_row(const uint16_t *cp, const double2 *v
 
 __global__ void __launch_bounds__(RT, 1)
 k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
-                const RsCta *__restrict__ ctas, const int2 *__restrict__ ucnt,
-                const int32_t *__restrict__ ulist, int umax, const uint16_t *__restrict__ scol,
-                const double2 *__restrict__ sval, int nbytes, int vsm, double rtol2, int max_iter,
+                const RsCta *__restrict__ ctas, int nbytes, double rtol2, int max_iter,
                 unsigned long long timeout_ns) {
     extern __shared__ __align__(128) unsigned char rs_area[];
     __shared__ CocgShared sh;
@@ -79,7 +77,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     double2 *xg = (double2 *)S.x, *x = xg + r0;
     double2 *pair = (double2 *)S.pair;   // (z, previous p) of row i at 2 i, 2 i + 1
     ulonglong2 *mail = S.mail;
-    const int nu = __ldg(&ucnt[blockIdx.x].x);
+    const int nu = __ldg(&S.ucnt[blockIdx.x].x);
     if (tid == 0) {
         memset(&sh.st, 0, sizeof(CocgState));
         sh.quit = 0;
@@ -96,7 +94,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     double2 *halo = (double2 *)area;
     area += (size_t)nu * 16;
     double2 *q, *r, *dinv;
-    if (vsm) {
+    if (S.vsm) {
         q = (double2 *)area;
         r = q + nloc;
         dinv = r + nloc;
@@ -110,7 +108,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     for (int i = tid; i <= nsl; i += RT) so[i] = (int)(__ldg(S.soff + me.sl0 + i) - off0);
     for (int i = tid; i < nsl << (5 - lsh); i += RT) perm[i] = __ldg(S.sperm + me.sl0 * 32 + i);
     for (int i = tid; i < nu; i += RT) {
-        const int32_t c = __ldg(ulist + (size_t)blockIdx.x * umax + i);
+        const int32_t c = __ldg(S.ulist + (size_t)blockIdx.x * S.umax + i);
         list[i] = c;
         if (c == (int32_t)r0) sh.own = i;
     }
@@ -128,8 +126,8 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     const int nres = sh.nres, eres = so[nres];
     double2 *mv = (double2 *)area;
     uint16_t *mc = (uint16_t *)(area + (size_t)eres * 16);
-    const uint16_t *gc = scol + off0;
-    const double2 *gv = sval + off0;
+    const uint16_t *gc = S.rcol + off0;
+    const double2 *gv = (const double2 *)S.rval + off0;
     for (int i = tid; i < eres; i += RT) mv[i] = __ldcs(gv + i);
     for (int i = tid; i < eres / 8; i += RT) ((int4 *)mc)[i] = __ldcs((const int4 *)gc + i);
     const double2 *pown = halo + sh.own;

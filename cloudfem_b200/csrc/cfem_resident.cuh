@@ -34,27 +34,22 @@
 // -> 19 us; Tet10 heat of 44,415 rows in FP32 45 -> 10.0 us; P1 heat of
 // 699,273 rows in FP64 (104 MB streamed per iteration at 5.2 TB/s) 60 -> 43 us.
 //
-// Sums depend on the system's own shape (block count, rows per block, lanes
-// per row), never on what else is in the batch, so a result is bitwise the
-// same alone and in a batch.
+// Sums depend on the system's own shape (block count, lanes per row), never
+// on what else is in the batch. There are two shapes, one for solves and a
+// denser one for solve slots (rs_shape); within either a result is bitwise the
+// same alone and in any batch.
 
 constexpr int RT = 512;              // threads per block
 constexpr int RWARPS = RT / 32;
 constexpr int RS_WINDOW = 256;       // rows sorted by length together
 constexpr int RS_SMEM_MAX = 224 * 1024;
 constexpr size_t RS_MAX_WAVES = 4;   // launches of one batch
+constexpr int RS_HOLD = 150 * 1024;  // matrix bytes a block is meant to hold
 constexpr int RS_COPIES = 8;         // copies of the partial sums, at most
 
 template <typename T> struct PairOf;
 template <> struct PairOf<float> { using type = float2; };
 template <> struct PairOf<double> { using type = double2; };
-
-// A block of the batch: its system, its number there, its rows and its
-// first slice in the batch's slice table.
-struct RsCta {
-    int32_t sys, cta, row0, rows;
-    int64_t sl0;
-};
 
 struct RsShared {
     double red[4][RWARPS];
@@ -198,52 +193,100 @@ __device__ __forceinline__ bool rs_sync(Shared &sh, ulonglong2 *mail, int nc, Gr
     return sh.quit == 0;
 }
 
-// U steps of one slice from step t on, loaded together; steps past the
-// slice's last repeat it with coefficient 0.
+// FP32 scalar slices keep a lane's slots in groups of Q = 4, so that a lane
+// loads a group's values in 16 bytes and its columns in 8: slot k of a lane
+// sits at 32 Q (k / Q) + Q lane + k % Q of the slice (widths are whole
+// groups). With one load per slot a streaming slice kept too little in flight:
+// 100,000 entries took a block 22 us, now 16. FP64 slots are one 8-byte load
+// each: pairs cost more in padding (P1 rows of 15) and registers than they gave.
+template <typename T> struct SlotGroup;
+template <> struct SlotGroup<float> {
+    static constexpr int Q = 4;
+    using V = float4;
+    using C = ushort4;
+};
+template <> struct SlotGroup<double> {
+    static constexpr int Q = 1;
+    using V = double;
+    using C = uint16_t;
+};
+// Slots per group of a slice's layout.
+__host__ __device__ inline int rs_group(int bs, size_t ts) { return bs == 1 && ts == 4 ? 4 : 1; }
+__device__ __forceinline__ int rs_slot(int k, int lane, int q) {
+    return 32 * q * (k / q) + q * lane + k % q;
+}
+__device__ __forceinline__ float4 ld_stream(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ ushort4 ld_stream(const ushort4 *p) {
+    ushort4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u16 {%0, %1, %2, %3}, [%4];"
+                 : "=h"(v.x), "=h"(v.y), "=h"(v.z), "=h"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void slots(const float4 &v, float o[4]) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+__device__ __forceinline__ void slots(double v, double o[1]) { o[0] = v; }
+__device__ __forceinline__ void slots(const ushort4 &v, int o[4]) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+__device__ __forceinline__ void slots(uint16_t v, int o[1]) { o[0] = v; }
+
+// Groups g .. g + U - 1 of a lane's slots, all loaded first; a group past the
+// n-th repeats the last (its values are not used): branches around the loads
+// instead cost the streaming FP64 rows a third of their rate.
 template <typename T, int U, bool SM>
-__device__ __forceinline__ void rs_load(const uint16_t *cp, const T *vp, int t, int w, int c[U],
-                                        T a[U]) {
+__device__ __forceinline__ void rs_load(const uint16_t *cp, const T *vp, int g, int n,
+                                        typename SlotGroup<T>::C c[U], typename SlotGroup<T>::V a[U]) {
+    using G = SlotGroup<T>;
 #pragma unroll
     for (int j = 0; j < U; ++j) {
-        const int tt = t + j < w ? t + j : w - 1;
-        c[j] = SM ? cp[32 * tt] : ld_stream(cp + 32 * tt);
+        const auto *p = (const typename G::C *)(cp + 32 * G::Q * (g + j < n ? g + j : n - 1));
+        c[j] = SM ? *p : ld_stream(p);
     }
 #pragma unroll
     for (int j = 0; j < U; ++j) {
-        const int tt = t + j < w ? t + j : w - 1;
-        a[j] = SM ? vp[32 * tt] : ld_stream(vp + 32 * tt);
+        const auto *p = (const typename G::V *)(vp + 32 * G::Q * (g + j < n ? g + j : n - 1));
+        a[j] = SM ? *p : ld_stream(p);
     }
-#pragma unroll
-    for (int j = 0; j < U; ++j) a[j] = t + j < w ? a[j] : (T)0;
 }
 
-// One lane's part of a row of a slice of 32 / L rows (L lanes per row):
-// slot k of a row sits at step k / L in lane k % L of the row's lanes; slot
-// 0 (diag: this lane holds it) is the diagonal, or the row sum of the FP32
-// difference form (DIFF), whose other slots multiply p_j - p_i.
-template <typename T, bool DIFF, int U, bool SM>
-__device__ __forceinline__ T rs_steps1(const uint16_t *cp, const T *vp, int t, int w, bool diag,
-                                       const T *halo, T pi) {
-    int c[U];
-    T a[U];
-    rs_load<T, U, SM>(cp, vp, t, w, c, a);
+// One lane's part of a row of a slice of 32 / L rows (L lanes per row, slot k
+// of the row in lane k % L); the row's slot 0 (diag: this lane holds it) is
+// the diagonal, or the row sum of the FP32 difference form (DIFF), whose
+// other slots multiply p_j - p_i. cp, vp: the lane's first group; w: slots.
+template <typename T, bool DIFF, bool SM, int U>
+__device__ __forceinline__ T rs_groups1(const uint16_t *cp, const T *vp, int g, int n, bool diag,
+                                        const T *halo, T pi) {
+    constexpr int Q = SlotGroup<T>::Q;
+    typename SlotGroup<T>::C c[U];
+    typename SlotGroup<T>::V a[U];
+    rs_load<T, U, SM>(cp, vp, g, n, c, a);
     T acc = 0;
 #pragma unroll
     for (int j = 0; j < U; ++j) {
-        T pj = halo[c[j]];
-        if (DIFF) pj = (diag && t + j == 0) ? pi : pj - pi;
-        acc += a[j] * pj;
+        int cj[Q];
+        T aj[Q];
+        slots(c[j], cj);
+        slots(a[j], aj);
+#pragma unroll
+        for (int e = 0; e < Q; ++e) {
+            T pj = halo[cj[e]];
+            if (DIFF) pj = (diag && g + j == 0 && e == 0) ? pi : pj - pi;
+            acc += (g + j < n ? aj[e] : (T)0) * pj;
+        }
     }
     return acc;
 }
-
-template <typename T, bool DIFF, bool SM>
+template <typename T, bool DIFF, bool SM, int SLOTS>
 __device__ __forceinline__ T rs_row1(const uint16_t *cp, const T *vp, int w, bool diag,
                                      const T *halo, T pi) {
+    constexpr int Q = SlotGroup<T>::Q, U = SLOTS / Q;
+    const int n = w / Q;
     T acc = 0;
-    int t = 0;
-    for (; w - t > 4; t += 8) acc += rs_steps1<T, DIFF, 8, SM>(cp, vp, t, w, diag, halo, pi);
-    if (t < w) acc += rs_steps1<T, DIFF, 4, SM>(cp, vp, t, w, diag, halo, pi);
+    int g = 0;
+    for (; n - g > U / 2; g += U) acc += rs_groups1<T, DIFF, SM, U>(cp, vp, g, n, diag, halo, pi);
+    if (g < n) acc += rs_groups1<T, DIFF, SM, U / 2>(cp, vp, g, n, diag, halo, pi);
     return acc;
 }
 
@@ -286,48 +329,52 @@ __device__ __forceinline__ void rs_row3(const uint16_t *cp, const T *vp, int w, 
 
 // Compensated sums of one lane's part of a row for the FP64 true residual
 // (x in the halo), with the sum of magnitudes for its round-off floor.
-template <int BS, bool SM>
-__device__ __forceinline__ void rs_row_dd(const uint16_t *cp, const double *vp, int w,
-                                          const double *halo, double hi[BS], double lo[BS],
-                                          double ab[BS]) {
-    constexpr int B2 = BS * BS, U = BS == 1 ? 4 : 1;
-    for (int t = 0; t < w; t += U) {
-        int c[U];
-        double a[U][B2];
+template <bool SM>
+__device__ __forceinline__ void rs_row_dd1(const uint16_t *cp, const double *vp, int w,
+                                           const double *halo, double &hi, double &lo, double &ab) {
+    constexpr int U = 4;
+    for (int g = 0; g < w; g += U) {
+        uint16_t c[U];
+        double a[U];
+        rs_load<double, U, SM>(cp, vp, g, w, c, a);
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-            const int tt = t + j < w ? t + j : w - 1;
-            c[j] = SM ? cp[32 * tt] : ld_stream(cp + 32 * tt);
+            if (g + j >= w) continue;
+            const double x0 = halo[c[j]];
+            dd_fma(hi, lo, a[j], x0);
+            ab += fabs(a[j] * x0);
         }
+    }
+}
+template <bool SM>
+__device__ __forceinline__ void rs_row_dd3(const uint16_t *cp, const double *vp, int w,
+                                           const double *halo, double hi[3], double lo[3],
+                                           double ab[3]) {
+    for (int t = 0; t < w; ++t) {
+        const int c = SM ? cp[32 * t] : ld_stream(cp + 32 * t);
+        double a[9];
 #pragma unroll
-        for (int j = 0; j < U; ++j) {
-            const int tt = t + j < w ? t + j : w - 1;
+        for (int e = 0; e < 9; ++e) a[e] = SM ? vp[32 * (9 * t + e)] : ld_stream(vp + 32 * (9 * t + e));
 #pragma unroll
-            for (int e = 0; e < B2; ++e)
-                a[j][e] = SM ? vp[32 * (B2 * tt + e)] : ld_stream(vp + 32 * (B2 * tt + e));
-        }
+        for (int d = 0; d < 3; ++d) {
+            const double xj = halo[3 * c + d];
 #pragma unroll
-        for (int j = 0; j < U; ++j) {
-            if (t + j >= w) continue;
-#pragma unroll
-            for (int d = 0; d < BS; ++d) {
-                const double xj = halo[BS * c[j] + d];
-#pragma unroll
-                for (int r = 0; r < BS; ++r) {
-                    dd_fma(hi[r], lo[r], a[j][r * BS + d], xj);
-                    ab[r] += fabs(a[j][r * BS + d] * xj);
-                }
+            for (int r = 0; r < 3; ++r) {
+                dd_fma(hi[r], lo[r], a[r * 3 + d], xj);
+                ab[r] += fabs(a[r * 3 + d] * xj);
             }
         }
     }
 }
 
+// list: (system, its block) of every block of the launch. A launch runs its
+// systems to the end, or for max_iters iterations when they may go on in a
+// later launch (keep: the residual and the Jacobi inverse then stay in
+// global memory between the launches; the rest is there anyway).
 template <typename T, int BS>
 __global__ void __launch_bounds__(RT, 1)
 k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
-           const RsCta *__restrict__ ctas, int first_cta, const int2 *__restrict__ ucnt,
-           const int32_t *__restrict__ ulist, int umax, const uint16_t *__restrict__ scol,
-           const T *__restrict__ sval, int nbytes, int vsm, int max_steps,
+           const int2 *__restrict__ list_, int nbytes, int max_steps, int max_iters, int keep,
            unsigned long long timeout_ns, unsigned hold) {
     extern __shared__ __align__(128) unsigned char rs_area[];
     __shared__ RsShared sh;
@@ -336,22 +383,27 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     constexpr bool DIFF = sizeof(T) == 4;
     constexpr int B2 = BS * BS;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int gcta = first_cta + blockIdx.x;
-    const RsCta me = ctas[gcta];
-    const int cta = me.cta;
+    const int2 place = __ldg(list_ + blockIdx.x);
+    const int cta = place.y;
     for (int i = tid; i < (int)(sizeof(SysDev) / 4); i += RT)
-        ((int *)&S)[i] = __ldg((const int *)(sys + me.sys) + i);
+        ((int *)&S)[i] = __ldcg((const int *)(sys + place.x) + i);
+    for (int i = tid; i < (int)(sizeof(SysState) / 4); i += RT)
+        ((int *)&sh.st)[i] = __ldcg((const int *)(gst + place.x) + i);
     if (tid == 0) {
-        memset(&sh.st, 0, sizeof(SysState));
         sh.quit = 0;
         sh.own = 0;
     }
     __syncthreads();
+    int ph = sh.st.phase;
+    if (ph == PH_DONE) return;
+    const RsCta me = S.ctas[cta];
+    const uint16_t *scol = S.rcol;
+    const T *sval = (const T *)S.rval;
     const int lsh = S.lsh, L = 1 << lsh;
     const int nloc = me.rows, nd = nloc * BS, nsl = rs_slices(nloc, lsh);
     const int64_t r0 = me.row0, d0 = r0 * BS;
     P2 *pair = (P2 *)S.pair;
-    const int nu = __ldg(&ucnt[gcta].x);
+    const int nu = __ldg(&S.ucnt[cta].x);
     // the block's own arrays
     unsigned char *area = rs_area;
     int *so = (int *)area;                       // slice offsets, from the block's first
@@ -364,13 +416,18 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     area += rs_al((size_t)nu * BS * sizeof(T));
     T *q, *r, *dinv;
     const uint8_t *fx;
-    if (vsm) {
+    if (S.vsm) {
         const size_t one = rs_al((size_t)nd * sizeof(T));
         q = (T *)area;
         r = (T *)(area + one);
         dinv = (T *)(area + 2 * one);
         uint8_t *f = area + 3 * one;
         for (int i = tid; i < nd; i += RT) f[i] = S.fixed ? __ldg(S.fixed + d0 + i) : 0;
+        if (ph != PH_INIT)
+            for (int i = tid; i < nd; i += RT) {
+                r[i] = __ldcg((const T *)S.r + d0 + i);
+                dinv[i] = __ldcg((const T *)S.dinv + d0 + i);
+            }
         fx = f;
         area += rs_vec_bytes(nloc, BS, sizeof(T));
     } else {
@@ -385,7 +442,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     for (int i = tid; i < nsl << (5 - lsh); i += RT)
         perm[i] = __ldg(S.sperm + me.sl0 * 32 + i);
     for (int i = tid; i < nu; i += RT) {
-        const int32_t c = __ldg(ulist + (size_t)gcta * umax + i);
+        const int32_t c = __ldg(S.ulist + (size_t)cta * S.umax + i);
         list[i] = c;
         if (c == (int32_t)r0) sh.own = i;        // own rows follow one another in the list
     }
@@ -416,8 +473,9 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     const T *pown = halo + (size_t)sh.own * BS;  // the direction on the block's own rows
     __syncthreads();
 
-    int ph = PH_INIT;
-    unsigned long long epoch = 0;
+    // the words of an earlier launch hold its epochs: go on from there
+    unsigned long long epoch = (unsigned long long)(unsigned)sh.st.pad;
+    const int iter0 = sh.st.iter;
     auto adv = [&](const double tot[4]) {
         if (ph == PH_INIT && tot[3] < 0.0) sh.st.status = CFEM_ERR_BREAKDOWN;
         advance(S, &sh.st, bar, ph, tot, cta == 0);
@@ -458,10 +516,9 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                     acc[c] = 0;
                 }
                 if constexpr (BS == 1) {
-                    acc[0] = s < nres ? rs_row1<T, DIFF, true>(mc + off + lane, mv + off + lane, w, first,
-                                                               halo, pi[0])
-                                      : rs_row1<T, DIFF, false>(gc + off + lane, gv + off + lane, w, first,
-                                                                halo, pi[0]);
+                    const int at = off + SlotGroup<T>::Q * lane;
+                    acc[0] = s < nres ? rs_row1<T, DIFF, true, 8>(mc + at, mv + at, w, first, halo, pi[0])
+                                      : rs_row1<T, DIFF, false, sizeof(T) == 4 ? 16 : 8>(gc + at, gv + at, w, first, halo, pi[0]);
                 } else {
                     if (s < nres)
                         rs_row3<T, DIFF, true>(mc + off + lane, mv + 9 * (size_t)off + lane, w, first,
@@ -535,12 +592,15 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                 double hi[BS], lo[BS], ab[BS];
 #pragma unroll
                 for (int c = 0; c < BS; ++c) hi[c] = lo[c] = ab[c] = 0.0;
-                if (s < nres)
-                    rs_row_dd<BS, true>(mc + off + lane, (const double *)mv + B2 * (size_t)off + lane, w, hx,
-                                        hi, lo, ab);
-                else
-                    rs_row_dd<BS, false>(gc + off + lane, (const double *)gv + B2 * (size_t)off + lane, w, hx,
-                                         hi, lo, ab);
+                if constexpr (BS == 1) {
+                    const int at = off + lane;
+                    if (s < nres) rs_row_dd1<true>(mc + at, (const double *)mv + at, w, hx, hi[0], lo[0], ab[0]);
+                    else rs_row_dd1<false>(gc + at, (const double *)gv + at, w, hx, hi[0], lo[0], ab[0]);
+                } else {
+                    const size_t at = 9 * (size_t)off + lane;
+                    if (s < nres) rs_row_dd3<true>(mc + off + lane, (const double *)mv + at, w, hx, hi, lo, ab);
+                    else rs_row_dd3<false>(gc + off + lane, (const double *)gv + at, w, hx, hi, lo, ab);
+                }
                 for (int o = L >> 1; o > 0; o >>= 1)
 #pragma unroll
                     for (int c = 0; c < BS; ++c) {
@@ -636,7 +696,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                         rz += (double)rv * (double)zv;
                         P2 g;
                         g.x = zv;
-                        g.y = init ? (T)0 : pown[i];
+                        g.y = init ? (T)0 : pair[d0 + i].y;
                         if (!init) s1 += (double)rv * (double)g.y;
                         pair[d0 + i] = g;
                     }
@@ -654,9 +714,18 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
         }
         if (!ok) return;
         ph = sh.st.phase;
-        if (ph == PH_DONE) break;
+        // (the update phase needs the product phase's vectors: not between)
+        if (ph == PH_DONE || (ph != PH_B && sh.st.iter - iter0 >= max_iters)) break;
     }
-    if (cta == 0 && tid == 0) gst[me.sys] = sh.st;
+    if (keep && S.vsm && ph != PH_DONE)
+        for (int i = tid; i < nd; i += RT) {
+            ((T *)S.r)[d0 + i] = r[i];
+            ((T *)S.dinv)[d0 + i] = dinv[i];
+        }
+    if (cta == 0 && tid == 0) {
+        sh.st.pad = (int32_t)epoch;
+        gst[place.x] = sh.st;
+    }
 }
 
 // ------------------------------------------------------------------ set-up
@@ -717,10 +786,10 @@ __global__ void k_rs_split(const SysDev *__restrict__ sys, RsCta *ctas, int n, i
 // Row order, slice sizes and halo size of every block: windows of RS_WINDOW
 // rows (the last one shorter) sorted by stored length, longest first, ties
 // in row order; a slice is 32 / L positions, its size 32 x its longest
-// row's slots rounded up to whole steps of L.
+// row's slots rounded up to whole steps of L and whole groups of q.
 __global__ void __launch_bounds__(RT)
 k_rs_rank(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int64_t *sizes_all,
-          int2 *ucnt) {
+          int2 *ucnt, int q) {
     extern __shared__ __align__(16) uint32_t rs_bits[];
     __shared__ int total;
     const RsCta me = ctas[blockIdx.x];
@@ -745,7 +814,7 @@ k_rs_rank(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int64_
         int rank = 0;
         for (int u = w0; u < w1; ++u) rank += (len[u] > Li || (len[u] == Li && u < i)) ? 1 : 0;
         perm[w0 + rank] = (uint8_t)(i - w0);
-        if (rank % rs == 0) sizes_all[me.sl0 + (w0 + rank) / rs] = 32 * (int64_t)((Li + L - 1) >> lsh);
+        if (rank % rs == 0) sizes_all[me.sl0 + (w0 + rank) / rs] = 32 * (int64_t)((((Li + L - 1) >> lsh) + q - 1) / q * q);
     }
     __syncthreads();
     if (t == 0) ucnt[blockIdx.x] = make_int2(total, me.rows);
@@ -771,8 +840,8 @@ __device__ __forceinline__ int rs_dpos(const int32_t *ci, int32_t kb, int len, i
 // Every block's halo list and the slices' local columns (places in that
 // list). A row repeated in the CSR keeps its repeats as entries.
 __global__ void __launch_bounds__(RT)
-k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int umax,
-          int32_t *__restrict__ ulist, uint16_t *__restrict__ scol) {
+k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas,
+          uint16_t *__restrict__ scol, int q) {
     extern __shared__ __align__(16) uint32_t rs_bits[];
     __shared__ int wsum[RWARPS];
     const RsCta me = ctas[blockIdx.x];
@@ -799,7 +868,7 @@ k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int um
     __syncthreads();
     int base = inc - sum;
     for (int k = 0; k < wid; ++k) base += wsum[k];
-    int32_t *list = ulist + (size_t)blockIdx.x * umax;
+    int32_t *list = (int32_t *)S.ulist + (size_t)me.cta * S.umax;
     for (int g = g0; g < g1; ++g) {
         pre[g] = base;
         for (int j = 0; j < 4; ++j) {
@@ -834,7 +903,7 @@ k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int um
         const uint16_t own = place((int32_t)(valid ? row : r0));
         for (int k = 0; k < w; ++k) {
             const int e = rs_entry(k * L + u, len, dpos);
-            scol[off + 32 * k + lane] = e >= 0 ? place(__ldg(S.ci + kb + e)) : own;
+            scol[off + rs_slot(k, lane, q)] = e >= 0 ? place(__ldg(S.ci + kb + e)) : own;
         }
     }
 }
@@ -844,7 +913,7 @@ k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, int um
 // padding. Run again when the values change.
 template <typename T, int BS>
 __global__ void __launch_bounds__(256)
-k_rs_vals(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, T *__restrict__ sval) {
+k_rs_vals(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, T *__restrict__ sval, int q) {
     constexpr int B2 = BS * BS;
     const RsCta me = ctas[blockIdx.x];
     const SysDev &S = sys[me.sys];
@@ -865,7 +934,7 @@ k_rs_vals(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas, T *__r
         const int dpos = rs_dpos(S.ci, kb, len, (int32_t)row, u, L);
         for (int k = 0; k < w; ++k) {
             const int e = rs_entry(k * L + u, len, dpos);
-            T *dst = sval + B2 * (off + 32 * (int64_t)k) + lane;
+            T *dst = BS == 1 ? sval + off + rs_slot(k, lane, q) : sval + B2 * (off + 32 * (int64_t)k) + lane;
 #pragma unroll
             for (int c = 0; c < B2; ++c)
                 dst[32 * c] = e >= 0 ? __ldg(v + ((int64_t)kb + e) * B2 + c) : T{};

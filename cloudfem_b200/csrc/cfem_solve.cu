@@ -64,6 +64,13 @@ constexpr int RS_MAX_CTAS = 160;           // blocks of one resident system, at 
 
 __host__ __device__ inline int chunk_rows(int bs) { return bs == 3 ? 8 : 16; }
 
+// A block of a resident batch: its system, its number there, its rows and
+// its first slice in the batch's slice table.
+struct RsCta {
+    int32_t sys, cta, row0, rows;
+    int64_t sl0;
+};
+
 struct SysDev {
     int64_t n;
     int32_t bs, precond, mode, max_iter;
@@ -115,9 +122,16 @@ struct SysDev {
     int32_t rsell;        // bs 1, mixed, A phase staged: an FP64 sliced-ELL copy
                           // (scol / sval / soff / sperm) for the residual phase
     // resident scheduler: blocks, log2 of the lanes per row, the system's
-    // place in the batch's slice table; (z, p) pairs and the partial sums
-    int32_t ncta, lsh;
+    // place in the batch's slice table; its blocks (rows, halo sizes and
+    // halos, umax entries apart), slice columns and values, whether the
+    // vectors sit in shared memory; (z, p) pairs and the partial sums
+    int32_t ncta, lsh, umax, vsm;
     int64_t sl0;
+    const RsCta *ctas;
+    const int2 *ucnt;
+    const int32_t *ulist;
+    const uint16_t *rcol;
+    const void *rval;
     void *pair;
     ulonglong2 *mail;
 };
@@ -3143,10 +3157,13 @@ struct cfem_pcg_plan {
     int max_iter = 1;
     bool persistent = true;
     bool resident = false;        // k_resident: `waves` launches of whole systems
-    std::vector<int2> waves;      // (first block, blocks) in the block table
+    bool rs_dense = false;        // ... in the batch shape
+    bool rs_keep = false;         // ... a solve slot: goes on over several launches
+    std::vector<int2> waves;      // (first block, blocks) in the launch list
+    int2 *rs_list = nullptr;      // launch list: (system, block)
     cfem::RsCta *d_ctas = nullptr;   // block table
     size_t rs_ts = 8;                // bytes of a vector entry (complex: 16)
-    int rs_ctas = 0, rs_smem = 0, rs_vsm = 0, rs_umax = 0;
+    int rs_ctas = 0, rs_smem = 0, rs_vsm = 0;
     int2 *rs_ucnt = nullptr;         // every block's halo size and rows
     int32_t *rs_ulist = nullptr;     // every block's halo
     char *rs_col = nullptr, *rs_val = nullptr;
@@ -3204,6 +3221,17 @@ struct cfem_pcg_plan {
     char *scan_tmp = nullptr;
     size_t scan_bytes = 0;
     int64_t *h_total = nullptr;
+    // slots on the resident kernel: each slot's system has a resident plan of
+    // its own (`sub`), all advanced by one launch per round over `rs_list`
+    std::vector<cfem_pcg_plan *> sub;
+    std::vector<char> rs_busy;        // the slot holds a resident system to advance
+    bool rs_dirty = true;             // rs_list is not that of rs_busy
+    int graph_busy = 0;               // slots whose systems run on the graphs
+    std::vector<char> on_graph;
+    char *rs_mem = nullptr;           // system table, states, barrier word, launch list
+    cfem::SysDev *rs_sys = nullptr;
+    cfem::SysState *rs_st = nullptr;
+    cfem::GridBar *rs_bar = nullptr;
     std::vector<cfem::SysDev> tmpl;   // slot templates: workspace pointers
     char *tmpl_mem = nullptr;         // the templates' placeholder CSR
     cudaGraph_t pgraph[2] = {nullptr, nullptr};
@@ -3409,6 +3437,14 @@ static int sell_layout(cfem_pcg_plan *P, cudaStream_t s) {
     return CFEM_OK;
 }
 
+// Memory of a slot's resident plan, after what is queued on w.
+static void rs_slot_free(cfem_pcg_plan *sub, cudaStream_t w) {
+    if (!sub) return;
+    for (char *m : {sub->ws_copy, sub->ws_state, sub->ws_sdata})
+        if (m) cudaFreeAsync(m, w);
+    delete sub;
+}
+
 static void plan_free(cfem_pcg_plan *P) {
     if (!P) return;
     cudaSetDevice(P->device);
@@ -3419,7 +3455,9 @@ static void plan_free(cfem_pcg_plan *P) {
         if (P->pexec[gi]) cudaGraphExecDestroy(P->pexec[gi]);
         if (P->pgraph[gi]) cudaGraphDestroy(P->pgraph[gi]);
     }
+    for (cfem_pcg_plan *sub : P->sub) rs_slot_free(sub, P->w);
     if (P->w) {
+        if (P->rs_mem) cudaFreeAsync(P->rs_mem, P->w);
         if (P->ws_copy) cudaFreeAsync(P->ws_copy, P->w);
         if (P->ws_state) cudaFreeAsync(P->ws_state, P->w);
         if (P->ws_smeta) cudaFreeAsync(P->ws_smeta, P->w);
@@ -3455,8 +3493,15 @@ static void plan_free(cfem_pcg_plan *P) {
 // box), more where a block has too few rows for its warps and the rows are
 // long (the phasor system's 90 entries); 3x3 block rows 4 lanes (20 and more blocks per row, Tet10) or 2 (27 x 15 x 13 Tet10 box in
 // FP32: 26.7 / 21.0 / 18.7 / 21.7 us per iteration for 1 / 2 / 4 / 8).
-static void rs_shape(int64_t n, int64_t nnzb, int bs, int num_sms, int &ncta, int &lsh) {
-    const int64_t per = bs == 3 ? 1024 : 2560;
+//
+// The dense shape, that of solve slots, gives a block as many entries as its
+// shared memory holds: several systems then run side by side instead of each
+// on the whole GPU (whose sums cost the same however little there is to add).
+// 24 served systems of 1,000 to 60,000 unknowns: 170 -> 38 ms against rounds of
+// captured launches over every slot's capacity.
+static void rs_shape(int64_t n, int64_t nnzb, int bs, size_t ts, bool dense, int num_sms, int &ncta,
+                     int &lsh) {
+    const int64_t per = dense ? RS_HOLD / (int64_t)(2 + bs * bs * ts) : (bs == 3 ? 1024 : 2560);
     ncta = (int)std::max<int64_t>(1, std::min<int64_t>((nnzb + per - 1) / per, num_sms));
     const int64_t mean = nnzb / n, rows = n / ncta;
     if (bs == 3) {
@@ -3480,19 +3525,28 @@ static size_t rs_map_bytes(int64_t n, int64_t rows, int lsh) {
 
 // Whether the batch may run on the resident scheduler, and its launches:
 // every system of one precision and block size, point Jacobi, the set-up's
-// column bitmap within shared memory, each launch as many whole systems as
-// the SMs hold blocks.
+// column bitmap within shared memory, as many whole systems to a launch as the
+// SMs hold blocks and at most RS_MAX_WAVES launches. A larger batch is the
+// graph scheduler's, whose launches share their latencies among all systems:
+// 48 Tet10 heat meshes of 4 to 24 cells (45 M entries) took 79 ms in the dense
+// shape, 64 ms with four times its entries per block, 58 ms as a graph.
 static bool rs_plan(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t *nnzb) {
+    const int sms = std::min(P->ctx->num_sms, RS_MAX_CTAS);
+    const size_t ts = systems[0].mode == CFEM_SOLVE_MIXED ? 4 : P->rs_ts;
     int used = 0, total = 0;
     P->waves.clear();
-    const int sms = std::min(P->ctx->num_sms, RS_MAX_CTAS);
     for (int i = 0; i < P->n_systems; ++i) {
         const cfem_linsys &L = systems[i];
-        if (L.bs != systems[0].bs || L.mode != systems[0].mode ||
+        if (L.bs != systems[0].bs || L.mode != systems[0].mode || nnzb[i] <= 0 ||
             (L.bs == 3 && L.precond != CFEM_PRECOND_JACOBI))
             return false;
+        // P1 elasticity in mixed precision keeps its former schedulers: at
+        // the default tolerance its answers still move by the rounding of the
+        // FP32 iteration (up to 1e-8 under thermal loads, any order of sums
+        // another 1e-9), Tet10 elasticity's by 1e-10 and less
+        if (L.bs == 3 && L.mode == CFEM_SOLVE_MIXED && nnzb[i] < 20 * L.n_rows) return false;
         int ncta, lsh;
-        rs_shape(L.n_rows, nnzb[i], L.bs, sms, ncta, lsh);
+        rs_shape(L.n_rows, nnzb[i], L.bs, ts, P->rs_dense, sms, ncta, lsh);
         if (rs_map_bytes(L.n_rows, rs_most_rows(L.n_rows, nnzb[i], L.bs, ncta), lsh) >
             (size_t)RS_SMEM_MAX)
             return false;
@@ -3512,7 +3566,8 @@ template <typename T, int BS>
 static int rs_vals(cfem_pcg_plan *P, cudaStream_t s) {
     const unsigned gy = (unsigned)std::max(1, std::min(16, P->ctx->num_sms * 8 / P->rs_ctas));
     (void)cudaGetLastError();
-    k_rs_vals<T, BS><<<dim3((unsigned)P->rs_ctas, gy), 256, 0, s>>>(P->d_sys, P->d_ctas, (T *)P->rs_val);
+    k_rs_vals<T, BS><<<dim3((unsigned)P->rs_ctas, gy), 256, 0, s>>>(P->d_sys, P->d_ctas, (T *)P->rs_val,
+                                                                       rs_group(BS, sizeof(T)));
     g_launches.fetch_add(1, std::memory_order_relaxed);
     CFEM_CUDA(cudaGetLastError());
     return CFEM_OK;
@@ -3579,7 +3634,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
         S.max_stall = L.max_stall > 0 ? L.max_stall : MAX_STALL;
         S.hist_cap = L.d_history ? L.history_cap : 0;
         S.hist = L.d_history;
-        rs_shape(L.n_rows, nnzb[i], bs, sms, S.ncta, S.lsh);
+        rs_shape(L.n_rows, nnzb[i], bs, ts, P->rs_dense, sms, S.ncta, S.lsh);
         S.sl0 = nslices;
         nslices += (S.n >> (5 - S.lsh)) + S.ncta + 1;
         for (int c = 0; c < S.ncta; ++c) ctas.push_back(RsCta{i, c, 0, 0, 0});
@@ -3587,14 +3642,17 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     }
     perm_bytes = align256((size_t)nslices * 32);
     P->rs_ctas = (int)ctas.size();
+    std::vector<int2> list;
+    for (const RsCta &c : ctas) list.push_back(make_int2(c.sys, c.cta));
     const size_t copy = align256(ns * sizeof(SysDev)) + align256(ctas.size() * sizeof(RsCta)) +
-                        perm_bytes + 2 * align256((nslices + 1) * 8) + align256(ctas.size() * 8);
+                        align256(list.size() * sizeof(int2)) + perm_bytes + 2 * align256((nslices + 1) * 8) + align256(ctas.size() * 8);
     CFEM_TRY(rs_alloc(P, &P->ws_copy, copy, s));
     if (!P->ws_copy) return CFEM_OK;
     size_t oc = 0;
     auto take_c = [&](size_t b) { char *p = P->ws_copy + oc; oc += align256(b); return (void *)p; };
     P->d_sys = (SysDev *)take_c(ns * sizeof(SysDev));
     P->d_ctas = (RsCta *)take_c(ctas.size() * sizeof(RsCta));
+    P->rs_list = (int2 *)take_c(list.size() * sizeof(int2));
     int64_t *sizes = (int64_t *)take_c((nslices + 1) * 8);
     int64_t *soff = (int64_t *)take_c((nslices + 1) * 8);
     P->rs_ucnt = (int2 *)take_c(ctas.size() * 8);
@@ -3606,12 +3664,15 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     CFEM_CUDA(cudaMemcpyAsync(P->d_sys, hs.data(), ns * sizeof(SysDev), cudaMemcpyHostToDevice, s));
     CFEM_CUDA(cudaMemcpyAsync(P->d_ctas, ctas.data(), ctas.size() * sizeof(RsCta),
                               cudaMemcpyHostToDevice, s));
+    CFEM_CUDA(cudaMemcpyAsync(P->rs_list, list.data(), list.size() * sizeof(int2),
+                              cudaMemcpyHostToDevice, s));
     CFEM_CUDA(cudaMemsetAsync(sizes, 0, (nslices + 1) * sizeof(int64_t), s));
     CFEM_LAUNCH(k_rs_split, grid_for(P->rs_ctas, 128), 128, 0, s, P->d_sys, P->d_ctas, P->rs_ctas,
                 rs_alpha(bs));
     CFEM_CUDA(cudaFuncSetAttribute(k_rs_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
     CFEM_CUDA(cudaFuncSetAttribute(k_rs_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
-    CFEM_LAUNCH(k_rs_rank, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas, sizes, P->rs_ucnt);
+    CFEM_LAUNCH(k_rs_rank, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas, sizes, P->rs_ucnt,
+                rs_group(bs, ts));
     size_t scan_bytes = 0;
     char *scan_tmp = nullptr;
     CFEM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, sizes, soff, nslices + 1, s));
@@ -3640,9 +3701,16 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     for (const SysDev &S : hs) {
         const size_t nd = (size_t)S.n * bs;
         state += align256(nd * 2 * ts) + align256(rs_mail_bytes(S.ncta)) +
-                 (P->rs_vsm ? 0 : 3 * align256(nd * ts));
+                 (P->rs_vsm && !P->rs_keep ? 0 : 3 * align256(nd * ts));
     }
-    const size_t ubytes = align256(ctas.size() * (size_t)umax * 4), cbytes = align256((size_t)total * 2);
+    // halo lists, as far apart as the system's longest
+    size_t lists = 0;
+    for (size_t c = 0, i = 0; i < hs.size(); c += hs[i++].ncta) {
+        hs[i].umax = 0;
+        for (int k = 0; k < hs[i].ncta; ++k) hs[i].umax = std::max(hs[i].umax, ucnt[c + k].x);
+        lists += (size_t)hs[i].ncta * hs[i].umax;
+    }
+    const size_t ubytes = align256(lists * 4), cbytes = align256((size_t)total * 2);
     bool take = umax <= 65535 && fixed <= (size_t)RS_SMEM_MAX;   // else too scattered a pattern
     if (take) {
         CFEM_TRY(rs_alloc(P, &P->ws_state, state, s));
@@ -3657,7 +3725,6 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     }
     P->resident = true;
     P->persistent = false;
-    P->rs_umax = umax;
     size_t os = 0;
     auto take_s = [&](size_t b) { char *p = P->ws_state + os; os += align256(b); return (void *)p; };
     P->d_st = (SysState *)take_s(ns * sizeof(SysState));
@@ -3667,18 +3734,29 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     for (SysDev &S : hs) {
         const size_t nd = (size_t)S.n * bs;
         S.pair = take_s(nd * 2 * ts);
-        if (!P->rs_vsm) {
+        if (!P->rs_vsm || P->rs_keep) {
             S.q = take_s(nd * ts);
             S.r = take_s(nd * ts);
             S.dinv = take_s(nd * ts);
         }
     }
-    CFEM_CUDA(cudaMemcpyAsync(P->d_sys, hs.data(), ns * sizeof(SysDev), cudaMemcpyHostToDevice, s));
     P->rs_ulist = (int32_t *)P->ws_sdata;
     P->rs_col = P->ws_sdata + ubytes;
     P->rs_val = P->rs_col + cbytes;
-    CFEM_LAUNCH(k_rs_cols, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas, umax,
-                P->rs_ulist, (uint16_t *)P->rs_col);
+    size_t c0 = 0, l0 = 0;
+    for (SysDev &S : hs) {
+        S.ctas = P->d_ctas + c0;
+        S.ucnt = P->rs_ucnt + c0;
+        S.ulist = P->rs_ulist + l0;
+        S.rcol = (const uint16_t *)P->rs_col;
+        S.rval = P->rs_val;
+        S.vsm = P->rs_vsm;
+        c0 += S.ncta;
+        l0 += (size_t)S.ncta * S.umax;
+    }
+    CFEM_CUDA(cudaMemcpyAsync(P->d_sys, hs.data(), ns * sizeof(SysDev), cudaMemcpyHostToDevice, s));
+    CFEM_LAUNCH(k_rs_cols, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas,
+                (uint16_t *)P->rs_col, rs_group(bs, ts));
     // shared memory: the vectors and, if it fits, the whole matrix with some
     // room for uneven blocks; the most where systems differ
     const size_t want = fixed + (size_t)total * (2 + (size_t)bs * bs * ts) / P->rs_ctas * 9 / 8 + 4096;
@@ -3689,18 +3767,24 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     return rs_copies(P, s);
 }
 
+// One launch of the resident kernel: blocks [first, first + n) of the list.
+static int rs_launch(cfem_pcg_plan *P, const SysDev *d_sys, SysState *d_st, GridBar *d_bar,
+                     const int2 *list, int n, int bs, int mode, int smem, int max_steps,
+                     int max_iters, cudaStream_t s) {
+    int keep = P->slots ? 1 : 0;
+    void *args[] = {(void *)&d_sys, (void *)&d_st, (void *)&d_bar, (void *)&list,
+                    (void *)&smem, (void *)&max_steps, (void *)&max_iters, (void *)&keep,
+                    (void *)&P->bar_timeout_ns, (void *)&P->bar_hold};
+    CFEM_CUDA(cudaLaunchCooperativeKernel(rs_kernel(bs, mode), dim3((unsigned)n), dim3(RT), args,
+                                          (size_t)smem, s));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return CFEM_OK;
+}
+
 static int rs_run(cfem_pcg_plan *P, cudaStream_t w) {
-    const SysDev &S = P->hs[0];
-    int max_steps = 3 * P->max_iter + 16;
-    for (const int2 &wave : P->waves) {
-        void *args[] = {(void *)&P->d_sys, (void *)&P->d_st, (void *)&P->d_bar, (void *)&P->d_ctas,
-                        (void *)&wave.x, (void *)&P->rs_ucnt, (void *)&P->rs_ulist, (void *)&P->rs_umax,
-                        (void *)&P->rs_col, (void *)&P->rs_val, (void *)&P->rs_smem,
-                        (void *)&P->rs_vsm, (void *)&max_steps, (void *)&P->bar_timeout_ns, (void *)&P->bar_hold};
-        CFEM_CUDA(cudaLaunchCooperativeKernel(rs_kernel(S.bs, S.mode), dim3((unsigned)wave.y),
-                                              dim3(RT), args, (size_t)P->rs_smem, w));
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-    }
+    for (const int2 &v : P->waves)
+        CFEM_TRY(rs_launch(P, P->d_sys, P->d_st, P->d_bar, P->rs_list + v.x, v.y, P->hs[0].bs,
+                           P->hs[0].mode, P->rs_smem, 3 * P->max_iter + 16, INT32_MAX, w));
     return CFEM_OK;
 }
 
@@ -3743,9 +3827,7 @@ int cocg_resident(cfem_ctx *ctx, int64_t n, const int32_t *ip, const int32_t *ix
         CocgState *d_st = (CocgState *)P.d_st;
         double rtol2 = rtol * rtol;
         void *args[] = {(void *)&P.d_sys, (void *)&d_st, (void *)&P.d_bar, (void *)&P.d_ctas,
-                        (void *)&P.rs_ucnt, (void *)&P.rs_ulist, (void *)&P.rs_umax,
-                        (void *)&P.rs_col, (void *)&P.rs_val, (void *)&P.rs_smem,
-                        (void *)&P.rs_vsm, (void *)&rtol2, (void *)&max_iter,
+                        (void *)&P.rs_smem, (void *)&rtol2, (void *)&max_iter,
                         (void *)&P.bar_timeout_ns};
         CFEM_CUDA(cudaEventRecord(e0, s));
         CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_resident_cocg, dim3((unsigned)P.rs_ctas),
@@ -3792,7 +3874,7 @@ static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,
     for (int i = 0; i < 2; ++i)
         for (int j = 0; j < 2; ++j) CFEM_CUDA(cudaEventCreate(&P->tev[i][j]));
     CFEM_CUDA(cudaMallocHost(&P->h_flags, 8 * sizeof(int)));
-    CFEM_CUDA(cudaMallocHost(&P->h_st, (size_t)n_systems * sizeof(SysState)));
+    CFEM_CUDA(cudaMallocHost(&P->h_st, (size_t)n_systems * (P->slots ? 2 : 1) * sizeof(SysState)));
     std::vector<SysDev> &hs = P->hs;
     hs.assign(n_systems, SysDev{});
     std::vector<int32_t> chunk_sys;
@@ -4479,6 +4561,22 @@ extern "C" int cfem_pcg_slots_create(cfem_ctx *ctx, int32_t n_slots, int32_t bs,
                 st = fail(CFEM_ERR_CUDA, "slot plan: events");
     }
     if (st == CFEM_OK) {
+        const size_t o_st = align256(n_slots * sizeof(SysDev));
+        const size_t o_bar = o_st + align256(n_slots * sizeof(SysState));
+        const size_t o_list = o_bar + align256(sizeof(GridBar));
+        const size_t bytes = o_list + align256((size_t)n_slots * RS_MAX_CTAS * sizeof(int2));
+        st = tmp_alloc(&P->rs_mem, bytes, P->w);
+        if (st == CFEM_OK && cudaMemsetAsync(P->rs_mem, 0, o_list, P->w) != cudaSuccess)
+            st = fail(CFEM_ERR_CUDA, "slot state reset failed");
+        P->rs_sys = (SysDev *)P->rs_mem;
+        P->rs_st = (SysState *)(P->rs_mem + o_st);
+        P->rs_bar = (GridBar *)(P->rs_mem + o_bar);
+        P->rs_list = (int2 *)(P->rs_mem + o_list);
+        P->sub.assign(n_slots, nullptr);
+        P->rs_busy.assign(n_slots, 0);
+        P->on_graph.assign(n_slots, 0);
+    }
+    if (st == CFEM_OK) {
         P->tmpl = P->hs;
         P->cap_rows.assign(n_slots, max_rows);
         P->cap_nnzb.assign(n_slots, max_nnzb);
@@ -4497,6 +4595,75 @@ extern "C" int cfem_pcg_slots_create(cfem_ctx *ctx, int32_t n_slots, int32_t bs,
     *out = P;
     return CFEM_OK;
     CFEM_API_END
+}
+
+// Puts a system into a slot on the resident kernel: a resident plan of its
+// own in the dense shape, its table entry and a zeroed state (the next round
+// begins with INIT). *taken false, and nothing changed, when its halo does
+// not fit.
+static int rs_assign(cfem_pcg_plan *P, int slot, const cfem_linsys *L, int32_t nnzb, cudaStream_t s,
+                     bool *taken) {
+    cfem_pcg_plan *sub = new cfem_pcg_plan();
+    sub->ctx = P->ctx;
+    sub->n_systems = 1;
+    sub->hs.assign(1, SysDev{});
+    sub->rs_dense = true;
+    sub->rs_keep = true;
+    int st = CFEM_OK;
+    if (rs_plan(sub, L, &nnzb)) st = rs_build(sub, L, &nnzb, s);
+    if (st != CFEM_OK || !sub->resident) {
+        rs_slot_free(sub, s);
+        return st;
+    }
+    cudaStream_t w = P->w;
+    auto put = [&]() -> int {
+        CFEM_CUDA(cudaMemsetAsync(sub->ws_state, 0, sub->state_bytes, s));
+        CFEM_CUDA(cudaEventRecord(P->ev[0], s));
+        CFEM_CUDA(cudaStreamWaitEvent(w, P->ev[0], 0));
+        CFEM_CUDA(cudaMemcpyAsync(P->rs_sys + slot, &sub->hs[0], sizeof(SysDev),
+                                  cudaMemcpyHostToDevice, w));
+        CFEM_CUDA(cudaMemsetAsync(P->rs_st + slot, 0, sizeof(SysState), w));
+        return CFEM_OK;
+    };
+    st = put();
+    if (st != CFEM_OK) {
+        rs_slot_free(sub, s);
+        return st;
+    }
+    rs_slot_free(P->sub[slot], w);    // after the rounds that read it
+    P->sub[slot] = sub;
+    P->rs_busy[slot] = 1;
+    P->rs_dirty = true;
+    *taken = true;
+    return CFEM_OK;
+}
+
+// One round of every resident slot: launches of whole systems, as many to a
+// launch as the SMs hold blocks.
+static int rs_round(cfem_pcg_plan *P, int iters, cudaStream_t w) {
+    if (P->rs_dirty) {
+        std::vector<int2> list;
+        P->waves.clear();
+        int smem = 0;
+        for (int i = 0; i < P->n_systems; ++i) {
+            if (!P->rs_busy[i]) continue;
+            const int n = P->sub[i]->hs[0].ncta;
+            if (P->waves.empty() || P->waves.back().y + n > std::min(P->ctx->num_sms, RS_MAX_CTAS))
+                P->waves.push_back(make_int2((int)list.size(), 0));
+            P->waves.back().y += n;
+            for (int c = 0; c < n; ++c) list.push_back(make_int2(i, c));
+            smem = std::max(smem, P->sub[i]->rs_smem);
+        }
+        P->rs_smem = smem;
+        if (!list.empty())
+            CFEM_CUDA(cudaMemcpyAsync(P->rs_list, list.data(), list.size() * sizeof(int2),
+                                      cudaMemcpyHostToDevice, w));
+        P->rs_dirty = false;
+    }
+    for (const int2 &v : P->waves)
+        CFEM_TRY(rs_launch(P, P->rs_sys, P->rs_st, P->rs_bar, P->rs_list + v.x, v.y, P->tmpl[0].bs,
+                           P->tmpl[0].mode, P->rs_smem, INT32_MAX, iters, w));
+    return CFEM_OK;
 }
 
 extern "C" int cfem_pcg_slots_assign(cfem_pcg_plan *P, int32_t slot, const cfem_linsys *L,
@@ -4562,6 +4729,19 @@ extern "C" int cfem_pcg_slots_assign(cfem_pcg_plan *P, int32_t slot, const cfem_
     CFEM_CHECK(!sell3 || *P->h_total <= P->cap_sell[slot], CFEM_ERR_INVALID,
                "system's sliced-ELL layout has %lld blocks, slot %d holds %lld",
                (long long)*P->h_total, slot, (long long)P->cap_sell[slot]);
+    if (P->on_graph[slot]) {          // the slot's last system, if the graphs had it
+        P->on_graph[slot] = 0;
+        --P->graph_busy;
+    }
+    if (T.bs == 1 || sell3) {
+        bool taken = false;
+        CFEM_TRY(rs_assign(P, slot, L, nnzb, s, &taken));
+        if (taken) return CFEM_OK;
+    }
+    P->rs_busy[slot] = 0;
+    P->rs_dirty = true;
+    P->on_graph[slot] = 1;
+    ++P->graph_busy;
     SysDev S = T;   // the slot's workspace, lists and copies
     if (sell3) {
         S.sperm = P->smeta[2 * slot + set].perm;
@@ -4616,7 +4796,8 @@ extern "C" int cfem_pcg_slots_run(cfem_pcg_plan *P, int32_t rounds, void *stream
     cudaStream_t s = (cudaStream_t)stream, w = P->w;
     CFEM_CUDA(cudaEventRecord(P->ev[0], s));
     CFEM_CUDA(cudaStreamWaitEvent(w, P->ev[0], 0));
-    for (int r = 0; r < rounds; ++r) {
+    CFEM_TRY(rs_round(P, POLL_ITERS * rounds, w));
+    for (int r = 0; r < rounds && P->graph_busy > 0; ++r) {
         CFEM_CUDA(cudaGraphLaunch(P->pexec[r & 1], w));
         g_launches.fetch_add((int64_t)P->per_iter * POLL_ITERS, std::memory_order_relaxed);
     }
@@ -4643,13 +4824,21 @@ extern "C" int cfem_pcg_slots_poll(cfem_pcg_plan *P, cfem_solve_stats *stats) {
     const int n = P->n_systems;
     CFEM_CUDA(cudaMemcpyAsync(P->h_st, P->d_st, n * sizeof(SysState),
                               cudaMemcpyDeviceToHost, P->w));
+    CFEM_CUDA(cudaMemcpyAsync(P->h_st + n, P->rs_st, n * sizeof(SysState),
+                              cudaMemcpyDeviceToHost, P->w));
     CFEM_CUDA(cudaMemcpyAsync(&P->h_flags[3], &P->d_bar->err, sizeof(int),
                               cudaMemcpyDeviceToHost, P->w));
+    CFEM_CUDA(cudaMemcpyAsync(&P->h_flags[4], &P->rs_bar->err, sizeof(int),
+                              cudaMemcpyDeviceToHost, P->w));
     CFEM_CUDA(cudaStreamSynchronize(P->w));
-    const SysState *hst = P->h_st;
     const int h_err = P->h_flags[3];
     for (int i = 0; i < n; ++i) {
         cfem_solve_stats &o = stats[i];
+        const SysState *hst = P->sub[i] && !P->on_graph[i] ? P->h_st + n : P->h_st;
+        if (P->rs_busy[i] && hst[i].phase == PH_DONE) {
+            P->rs_busy[i] = 0;
+            P->rs_dirty = true;
+        }
         memset(&o, 0, sizeof(o));
         o.status = hst[i].phase == PH_DONE ? hst[i].status : CFEM_SLOT_RUNNING;
         o.iterations = hst[i].iter;
@@ -4659,6 +4848,8 @@ extern "C" int cfem_pcg_slots_poll(cfem_pcg_plan *P, cfem_solve_stats *stats) {
     }
     CFEM_CHECK(h_err != 2, CFEM_ERR_TIMEOUT,
                "solver SpMV bulk-copy wait timed out (device wait bound reached)");
+    CFEM_CHECK(P->h_flags[4] == 0, CFEM_ERR_TIMEOUT,
+               "solver grid barrier timed out (device wait bound reached)");
     return CFEM_OK;
     CFEM_API_END
 }
@@ -4671,6 +4862,9 @@ extern "C" int cfem_pcg_slots_release(cfem_pcg_plan *P, int32_t slot, void *stre
     cudaStream_t s = (cudaStream_t)stream, w = P->w;
     CFEM_CUDA(cudaEventRecord(P->ev[0], s));
     CFEM_CUDA(cudaStreamWaitEvent(w, P->ev[0], 0));
+    P->rs_busy[slot] = 0;
+    P->rs_dirty = true;
+    CFEM_LAUNCH(k_slot_cancel, 1, 32, 0, w, P->rs_st + slot, P->rs_bar);
     CFEM_LAUNCH(k_slot_cancel, 1, 32, 0, w, P->d_st + slot, P->d_bar);
     CFEM_CUDA(cudaEventRecord(P->ev[1], w));
     CFEM_CUDA(cudaStreamWaitEvent(s, P->ev[1], 0));

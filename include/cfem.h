@@ -487,19 +487,21 @@ CFEM_API int cfem_pcg_plan_destroy(cfem_pcg_plan *plan);
  * where systems arrive while others are being solved (the reference solves
  * one call at a time and has no counterpart). A slot plan holds n_slots
  * systems of one block size (1 or 3) and precision mode, each of at most
- * max_rows block rows and max_nnzb stored blocks, with point Jacobi; its
- * work lists, workspace and iteration graphs are fixed at creation. Assign
- * puts a system into a free slot (its working copy built, its state reset,
- * INIT run: it joins whatever is running), run queues `rounds` replays of
- * 16 iterations over every slot on the plan's stream (idle slots cost an
- * early exit), poll waits for the plan's stream and reports every slot
- * (status CFEM_SLOT_RUNNING while a system iterates; a finished system keeps
- * its status until the slot is assigned again), ready returns CFEM_OK once
- * the queued rounds have run and CFEM_SLOT_RUNNING before (no wait), release
- * ends a running system or frees a finished one. 3x3 slots hold the
- * sliced-ELL layout by default (CFEM_PARAM_SLOT_SELL3): assign then also
- * refuses (CFEM_ERR_INVALID, nothing changed) a system whose layout exceeds
- * the slot's room, which a block row of more than 96 blocks can cause.
+ * max_rows block rows and max_nnzb stored blocks, with point Jacobi. Assign
+ * puts a system into a free slot (its working copy built, its state reset: it
+ * joins whatever is running), run queues `rounds` rounds of 16 iterations
+ * over every slot on the plan's stream, poll waits for the plan's stream and
+ * reports every slot (status CFEM_SLOT_RUNNING while a system iterates; a
+ * finished system keeps its status until the slot is assigned again), ready
+ * returns CFEM_OK once the queued rounds have run and CFEM_SLOT_RUNNING
+ * before (no wait), release ends a running system or frees a finished one.
+ * Systems run on the resident kernel, one launch per round over the busy
+ * slots; those it does not take (a pattern too scattered for its halo, 3x3
+ * systems with CFEM_PARAM_SLOT_SELL3 0) on captured graphs over the slots'
+ * capacity. 3x3 slots size their copy for the sliced-ELL layout by default
+ * (CFEM_PARAM_SLOT_SELL3): assign then refuses (CFEM_ERR_INVALID, nothing
+ * changed) a system whose layout exceeds the slot's room, which a block row
+ * of more than 96 blocks can cause.
  * The caller keeps a system's arrays alive
  * while it is in a slot and reads x after poll reports it finished. Each
  * system's scalars and sums are its own, so its iterates do not depend on

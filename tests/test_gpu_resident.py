@@ -32,6 +32,8 @@ def _pattern(n, kind, rng):
     if kind == "band":
         d = [o for o in (1, 2, 7, 40) if o < n]
         P = sp.diags([np.ones(n - o) for o in d] + [np.ones(n)], d + [0], format="coo")
+    elif kind == "wide":           # 21 and more entries per row (Tet10-like)
+        P = sp.diags([np.ones(n - o) for o in range(min(12, n))], range(min(12, n)), format="coo")
     elif kind == "arrow":          # one row and column with every entry
         P = sp.coo_matrix((np.ones(n), (np.zeros(n, int), np.arange(n))), shape=(n, n))
         P = P + sp.identity(n) + sp.diags([np.ones(n - 1)], [1])
@@ -84,7 +86,8 @@ def _block_system(torch, rt, data, bs):
 
 
 SHAPES = [(1, "band"), (31, "band"), (33, "band"), (300, "band"), (257, "arrow"), (2561, "band"),
-          (6000, "arrow"), (5000, "scatter"), (40000, "band"), (150001, "band"), (100000, "scatter")]
+          (6000, "arrow"), (5000, "scatter"), (40000, "band"), (150001, "band"), (100000, "scatter"),
+          (9000, "wide"), (30000, "wide")]
 
 
 @pytest.mark.parametrize("bs", [1, 3])
@@ -123,8 +126,8 @@ def test_batch_of_several_launches_equals_alone(torch, bs):
     from cloudfem_b200 import _native as N
     from cloudfem_b200.device import pcg
     rt = N.runtime()
-    sizes = (5, 9000, 700, 30000, 64)
-    datas = [_system(n, bs, "band", n + bs) for n in sizes]
+    sizes = (70, 9000, 700, 30000)
+    datas = [_system(n, bs, "wide", n + bs) for n in sizes]
     for mode, rtol in ((N.SOLVE_FP64, 1e-13), (N.SOLVE_MIXED, 1e-10)):
         systems = [_block_system(torch, rt, d, bs) for d in datas]
         rb = pcg(systems, mode, rtol, 2000)
@@ -206,3 +209,56 @@ def test_cocg_matches_direct(torch, n, kind):
     if kind != "scatter":
         ref = spla.spsolve(A.tocsc(), b)
         assert np.linalg.norm(xs - ref) <= 1e-10 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("bs", [1, 3])
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_slots_go_on_over_rounds(torch, mode, bs):
+    """Systems of one block and of many in solve slots, advanced 16 iterations
+    a round (state, residual and inverse kept between launches), one released
+    on the way and its slot taken again: each answer bitwise that of a slot
+    engine of its own, and within the solve tolerance of the direct one
+    (tolerances as above)."""
+    from cloudfem_b200 import _native as N
+    from cloudfem_b200.device import SlotEngine
+    rt = N.runtime()
+    md, rtol, tol = ((N.SOLVE_FP64, 1e-13, 1e-12) if mode == "fp64" else (N.SOLVE_MIXED, 1e-10, 1e-9))
+    sizes = (3, 40, 4000, 12000)
+    datas = [_system(n, bs, "wide", n) for n in sizes]
+    cap = max(sizes)
+    make = lambda d: _block_system(torch, rt, d, bs)  # noqa: E731
+    eng = SlotEngine(rt, 3, bs, md, cap, cap * 30)
+    done = {}
+
+    def round_(engine):
+        engine.run(1)
+        for system, tag, res in engine.poll():
+            assert res.status == N.CFEM_OK, (tag, res)
+            done[tag] = system.x.clone()
+
+    def drain(engine, want):
+        for _ in range(400):
+            if all(t in done for t in want):
+                return
+            round_(engine)
+        raise AssertionError("slots did not finish")
+
+    first = eng.assign(make(datas[3]), rtol, 2000, tag="gone")
+    eng.assign(make(datas[0]), rtol, 2000, tag=0)
+    round_(eng)
+    eng.release(first)
+    for i in (1, 2):
+        eng.assign(make(datas[i]), rtol, 2000, tag=i)
+    drain(eng, (0, 1, 2))
+    eng.assign(make(datas[3]), rtol, 2000, tag=3)
+    drain(eng, (3,))
+    got = dict(done)
+    for i, d in enumerate(datas):
+        one = SlotEngine(rt, 1, bs, md, cap, cap * 30)
+        one.assign(make(d), rtol, 2000, tag=("alone", i))
+        drain(one, (("alone", i),))
+        assert torch.equal(done[("alone", i)], got[i]), i
+        x = _exact(d[0], d[4], d[5], d[6])
+        assert np.linalg.norm(got[i].cpu().numpy() - x) <= tol * np.linalg.norm(x)
+        one.close()
+    eng.close()
