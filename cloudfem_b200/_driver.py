@@ -67,7 +67,7 @@ def solve_block(dm, bs, vals, rhs, fixed_idx, fixed_val, precision="fp64",
     n = dm.n_nodes * bs
     mask, x = fixed_mask(dm.rt, n, fixed_idx, fixed_val, x0)
     sysm = BlockSystem(dm.rt, dm.n_nodes, bs, pat.row_ptr, pat.col, vals, rhs,
-                       x, mask)
+                       x, mask, nodes=dm.nodes if bs == 3 else None)
     res = pcg([sysm], mode, rtol, max_iter)
     _record(res)
     accept(res[0], rtol, what)

@@ -140,6 +140,8 @@ SIGNATURES = [
     ("cfem_mixed_matrix_batch", ctypes.c_int, [_vp, ctypes.POINTER(MixedJob), _i32, _vp]),
     ("cfem_pcg_solve", ctypes.c_int,
      [_vp, ctypes.POINTER(LinSys), _i32, ctypes.POINTER(SolveStats), _vp]),
+    ("cfem_pcg_solve_nodes", ctypes.c_int,
+     [_vp, ctypes.POINTER(LinSys), _vp, ctypes.POINTER(SolveStats), _vp]),
     ("cfem_pcg_plan_create", ctypes.c_int,
      [_vp, ctypes.POINTER(LinSys), ctypes.c_int32, _vp, ctypes.POINTER(_vp)]),
     ("cfem_pcg_plan_refresh", ctypes.c_int, [_vp, _vp]),

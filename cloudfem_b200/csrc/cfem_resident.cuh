@@ -46,6 +46,7 @@ constexpr int RS_SMEM_MAX = 224 * 1024;
 constexpr size_t RS_MAX_WAVES = 4;   // launches of one batch
 constexpr int RS_HOLD = 150 * 1024;  // matrix bytes a block is meant to hold
 constexpr int RS_COPIES = 8;         // copies of the partial sums, at most
+constexpr int RM = 6;                // rigid-body modes of a piece (cfem_coarse.cuh)
 
 template <typename T> struct PairOf;
 template <> struct PairOf<float> { using type = float2; };
@@ -57,6 +58,11 @@ struct RsShared {
     int quit;
     int nres;                        // leading slices held in shared memory
     int own;                         // place of the block's first row in its halo
+};
+// ... of the coarse correction: partial sums, products with the coarse
+// inverse, the block's own coefficients y
+struct RsCoarse {
+    double red[RM][64], prod[2][RM], y[RM];
 };
 
 __host__ __device__ inline size_t rs_al(size_t v) { return (v + 15) & ~(size_t)15; }
@@ -72,6 +78,11 @@ __host__ __device__ inline size_t rs_meta_bytes(int rows, int lsh) {
 }
 __host__ __device__ inline size_t rs_halo_bytes(int u, int bs, size_t ts) {
     return rs_al((size_t)u * 4) + rs_al((size_t)u * bs * ts);
+}
+// ... of the coarse correction: the block's rows of the coarse inverse, the
+// sums of all pieces, the rows' coordinates in their piece.
+__host__ __device__ inline size_t rs_coarse_bytes(int rows, int ncta) {
+    return (size_t)(RM + 1) * RM * ncta * 8 + rs_al((size_t)rows * 12);
 }
 __host__ __device__ inline size_t rs_vec_bytes(int rows, int bs, size_t ts) {
     const size_t nd = (size_t)rows * bs;
@@ -371,7 +382,8 @@ __device__ __forceinline__ void rs_row_dd3(const uint16_t *cp, const double *vp,
 // systems to the end, or for max_iters iterations when they may go on in a
 // later launch (keep: the residual and the Jacobi inverse then stay in
 // global memory between the launches; the rest is there anyway).
-template <typename T, int BS>
+// CO: with the coarse correction of cfem_coarse.cuh.
+template <typename T, int BS, bool CO = false>
 __global__ void __launch_bounds__(RT, 1)
 k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
            const int2 *__restrict__ list_, int nbytes, int max_steps, int max_iters, int keep,
@@ -379,6 +391,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     extern __shared__ __align__(128) unsigned char rs_area[];
     __shared__ RsShared sh;
     __shared__ SysDev S;
+    __shared__ typename std::conditional<CO, RsCoarse, int>::type co;
     using P2 = typename PairOf<T>::type;
     constexpr bool DIFF = sizeof(T) == 4;
     constexpr int B2 = BS * BS;
@@ -436,6 +449,17 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
         dinv = (T *)S.dinv + d0;
         fx = S.fixed ? S.fixed + d0 : nullptr;
     }
+    double *ainv = nullptr, *gall = nullptr;     // coarse inverse (own rows), all pieces' sums
+    float *xl = nullptr;
+    const int nm = RM * S.ncta;
+    if constexpr (CO) {
+        ainv = (double *)area;
+        gall = ainv + RM * nm;
+        xl = (float *)(gall + nm);
+        area += rs_coarse_bytes(nloc, S.ncta);
+        for (int i = tid; i < RM * nm; i += RT) ainv[i] = __ldg(S.ainv + (size_t)RM * cta * nm + i);
+        for (int i = tid; i < 3 * nloc; i += RT) xl[i] = __ldg(S.xl + 3 * r0 + i);
+    }
     const int64_t *gso = S.soff + me.sl0;
     const int64_t off0 = __ldg(gso);
     for (int i = tid; i <= nsl; i += RT) so[i] = (int)(__ldg(gso + i) - off0);
@@ -480,10 +504,90 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
         if (ph == PH_INIT && tot[3] < 0.0) sh.st.status = CFEM_ERR_BREAKDOWN;
         advance(S, &sh.st, bar, ph, tot, cta == 0);
     };
+    // Coarse correction: w += R_i^T v for a row's vector v (0 at fixed DOFs);
+    // the block's sums of w to its place among all pieces'; after the grid has
+    // met, the block's six products with the coarse inverse in co.prod.
+    auto mode_add = [&](double w[RM], int rl, const double v[3]) {
+        const double x = xl[3 * rl], y = xl[3 * rl + 1], z = xl[3 * rl + 2];
+        w[0] += v[0];
+        w[1] += v[1];
+        w[2] += v[2];
+        w[3] += y * v[2] - z * v[1];
+        w[4] += z * v[0] - x * v[2];
+        w[5] += x * v[1] - y * v[0];
+    };
+    auto modes_out = [&](double w[RM]) {
+        if constexpr (CO) {
+#pragma unroll
+            for (int k = 0; k < RM; ++k) {
+#pragma unroll
+                for (int o = 16; o > 2; o >>= 1) w[k] += __shfl_xor_sync(0xffffffffu, w[k], o);
+                if (lane < 4) co.red[k][4 * wid + lane] = w[k];
+            }
+            __syncthreads();
+            if (wid < RM) {
+                const double t = warp_sum(co.red[wid][lane] + co.red[wid][lane + 32]);
+                if (lane == 0) S.gall[RM * cta + wid] = t;
+            }
+        }
+    };
+    auto modes_in = [&]() {
+        if constexpr (CO) {
+            for (int i = tid; i < nm; i += RT) gall[i] = __ldcg(S.gall + i);
+            __syncthreads();
+            if (wid < 2 * RM) {
+                const int k = wid % RM;
+                double t = 0.0;
+                for (int i = (wid / RM) * 32 + lane; i < nm; i += 64) t += ainv[k * nm + i] * gall[i];
+                t = warp_sum(t);
+                if (lane == 0) co.prod[wid / RM][k] = t;
+            }
+            __syncthreads();
+        }
+    };
+    // (P y)_i of DOF c of a row
+    auto coarse_at = [&](int rl, int c) -> double {
+        if constexpr (CO) {
+            const double x = xl[3 * rl], y = xl[3 * rl + 1], z = xl[3 * rl + 2];
+            const double *a = co.y;
+            return c == 0 ? a[0] + z * a[4] - y * a[5]
+                          : (c == 1 ? a[1] - z * a[3] + x * a[5] : a[2] + y * a[3] - x * a[4]);
+        }
+        return 0.0;
+    };
+    // After a true residual: its coarse sums over the grid, the block's y, then
+    // z and the direction's partner on its rows; returns r.z (ok: no wait
+    // gave up).
+    auto coarse_residual = [&](double w[RM], bool init, bool &ok) -> double {
+        double rz = 0.0;
+        if constexpr (CO) {
+            modes_out(w);
+            double none[4] = {0.0, 0.0, 0.0, 0.0};
+            ok = rs_sync<1, true>(sh, S.mail, S.ncta, bar, cta, epoch, none, timeout_ns, hold,
+                                  [](const double *) {});
+            ++epoch;
+            if (!ok) return 0.0;
+            modes_in();
+            if (tid < RM) co.y[tid] = co.prod[0][tid] + co.prod[1][tid];
+            __syncthreads();
+            for (int i = tid; i < nd; i += RT) {
+                const int rl = i / 3;
+                const bool fixed = fx && fx[i];
+                const T rv = r[i];
+                P2 g;
+                g.x = fixed ? (T)0 : (T)((double)(dinv[i] * rv) + coarse_at(rl, i - 3 * rl));
+                g.y = init ? (T)0 : pair[d0 + i].y;
+                pair[d0 + i] = g;
+                rz += (double)rv * (double)g.x;
+            }
+        }
+        return rz;
+    };
     for (int step = 0; step < max_steps; ++step) {
         double part[4] = {0.0, 0.0, 0.0, 0.0};
+        double wm[RM] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         ++epoch;
-        bool ok;
+        bool ok = true;
         if (ph == PH_A) {
             const T beta = (T)sh.st.beta, zeta = (T)sh.st.zeta;
             const int nh = nu * BS;
@@ -536,10 +640,23 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                         q[rl * BS + c] = acc[c];
                         pq += (double)pi[c] * (double)acc[c];
                     }
+                    if constexpr (CO) {
+                        double v[3];
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) v[c] = fx && fx[rl * 3 + c] ? 0.0 : (double)acc[c];
+                        mode_add(wm, rl, v);
+                    }
                 }
             }
             part[0] = pq;
-            ok = rs_sync<1, false>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
+            if constexpr (CO) modes_out(wm);
+            ok = rs_sync<1, CO>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
+            if (CO && ok && sh.st.phase == PH_B) {   // y follows the residual
+                modes_in();
+                if constexpr (CO)
+                    if (tid < RM) co.y[tid] -= sh.st.alpha * (co.prod[0][tid] + co.prod[1][tid]);
+                __syncthreads();
+            }
         } else if (ph == PH_B) {
             const double alpha64 = sh.st.alpha;
             const T alpha = (T)alpha64;
@@ -554,7 +671,9 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                     rv -= alpha * q[i];
                     r[i] = rv;
                 }
-                const T zv = fixed ? (T)0 : dinv[i] * rv;
+                T zv = dinv[i] * rv;
+                if constexpr (CO) zv = (T)((double)zv + coarse_at(i / 3, i % 3));
+                if (fixed) zv = (T)0;
                 P2 g;
                 g.x = zv;
                 g.y = pi;
@@ -620,12 +739,22 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                         const T rv = (T)rt;
                         r[i] = rv;
                         P2 g = pair[d0 + i];
-                        g.x = fixed ? (T)0 : dinv[i] * rv;
-                        pair[d0 + i] = g;
-                        rz += (double)rv * (double)g.x;
                         rp += (double)rv * (double)g.y;
+                        if (!CO) {
+                            g.x = fixed ? (T)0 : dinv[i] * rv;
+                            pair[d0 + i] = g;
+                            rz += (double)rv * (double)g.x;
+                        }
+                    }
+                    if constexpr (CO) {
+                        const double v[3] = {(double)r[3 * rl], (double)r[3 * rl + 1], (double)r[3 * rl + 2]};
+                        mode_add(wm, rl, v);
                     }
                 }
+            }
+            if constexpr (CO) {
+                rz = coarse_residual(wm, false, ok);
+                if (!ok) return;
             }
             part[0] = rr;
             part[1] = rp;
@@ -692,15 +821,24 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                         } else {
                             dv = dinv[i];
                         }
-                        const T zv = fixed ? (T)0 : dv * rv;
-                        rz += (double)rv * (double)zv;
                         P2 g;
-                        g.x = zv;
                         g.y = init ? (T)0 : pair[d0 + i].y;
                         if (!init) s1 += (double)rv * (double)g.y;
-                        pair[d0 + i] = g;
+                        if (!CO) {
+                            g.x = fixed ? (T)0 : dv * rv;
+                            rz += (double)rv * (double)g.x;
+                            pair[d0 + i] = g;
+                        }
+                    }
+                    if constexpr (CO) {
+                        const double v[3] = {(double)r[3 * rl], (double)r[3 * rl + 1], (double)r[3 * rl + 2]};
+                        mode_add(wm, rl, v);
                     }
                 }
+            }
+            if constexpr (CO) {
+                rz = coarse_residual(wm, init, ok);
+                if (!ok) return;
             }
             part[0] = rr;
             part[1] = s1;

@@ -398,7 +398,7 @@ class BlockSystem:
     """One SPD block-CSR system on the device, ready for cfem_pcg_solve."""
 
     def __init__(self, rt, n_rows, bs, row_ptr, col, vals64, b, x,
-                 fixed=None, vals32=None, precond=None, keep=()):
+                 fixed=None, vals32=None, precond=None, keep=(), nodes=None):
         self.rt = rt
         self.n_rows = n_rows
         self.bs = bs
@@ -415,6 +415,9 @@ class BlockSystem:
         self.precond = (precond if precond is not None else
                         N.PRECOND_JACOBI)
         self.keep = keep
+        # (n_rows, 3) device coordinates of a 3x3 system's nodes, if known:
+        # lets pcg() of the system alone use their rigid-body modes
+        self.nodes = nodes
 
     def ensure_fp32(self):
         """FP32 difference-form operator for the mixed solver."""
@@ -462,8 +465,12 @@ def pcg(systems, mode=N.SOLVE_FP64, rtol=1e-12, max_iter=None,
         arr[i] = s.linsys(mode, rtol, mi, reliable_delta, max_stall,
                           None if history is None else history[i])
     stats = (N.SolveStats * len(systems))()
-    N.check(rt.lib.cfem_pcg_solve(rt.ctx, arr, len(systems), stats,
-                                  rt.stream()))
+    if len(systems) == 1 and systems[0].nodes is not None:
+        N.check(rt.lib.cfem_pcg_solve_nodes(rt.ctx, arr, ptr(systems[0].nodes), stats,
+                                            rt.stream()))
+    else:
+        N.check(rt.lib.cfem_pcg_solve(rt.ctx, arr, len(systems), stats,
+                                      rt.stream()))
     return [SolveResult(s) for s in stats]
 
 

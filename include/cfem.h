@@ -464,6 +464,19 @@ CFEM_API int cfem_mixed_matrix_batch(cfem_ctx *ctx, const cfem_mixed_job *jobs,
 CFEM_API int cfem_pcg_solve(cfem_ctx *ctx, const cfem_linsys *systems,
                    int32_t n_systems, cfem_solve_stats *stats, void *stream);
 
+/* cfem_pcg_solve for ONE 3x3 system whose block rows are mesh nodes with
+ * coordinates d_nodes (n_rows x 3, device; NULL: cfem_pcg_solve). With the
+ * geometry known, point Jacobi is complemented by a coarse correction on the
+ * rigid-body modes of pieces of the mesh (cfem_coarse.cuh), which takes
+ * several times fewer iterations on elasticity; the answer meets the same
+ * tolerance. Systems it is not for (other block sizes or preconditioners, a
+ * history asked for, fewer than 2,048 stored blocks, another scheduler than
+ * AUTO, a layout that does not fit) and solves that do not converge with it
+ * are those of cfem_pcg_solve. Used by solve_elasticity_* (elastic3d.py:230,
+ * elastic_tet10.py:228). Synchronises. */
+CFEM_API int cfem_pcg_solve_nodes(cfem_ctx *ctx, const cfem_linsys *system, const double *d_nodes,
+                                  cfem_solve_stats *stats, void *stream);
+
 /* Solve plans: the set-up of cfem_pcg_solve kept for repeated solves of the
  * same systems (time steps, serving), as spla.factorized is kept by
  * tet_heat.py:254 and tet10.py:524. Create captures the systems' device
