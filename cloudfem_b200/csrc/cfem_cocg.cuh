@@ -92,7 +92,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     int32_t *list = (int32_t *)area;
     area += rs_al((size_t)nu * 4);
     double2 *halo = (double2 *)area;
-    area += (size_t)nu * 16;
+    area += (size_t)((nu + 31) & ~31) * 16;
     double2 *q, *r, *dinv;
     if (S.vsm) {
         q = (double2 *)area;
@@ -130,14 +130,14 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     const double2 *gv = (const double2 *)S.rval + off0;
     for (int i = tid; i < eres; i += RT) mv[i] = __ldcs(gv + i);
     for (int i = tid; i < eres / 8; i += RT) ((int4 *)mc)[i] = __ldcs((const int4 *)gc + i);
-    const double2 *pown = halo + sh.own;
+    const int own = sh.own;
     __syncthreads();
 
     // q = A (halo) on the block's rows; fin(row, value, diagonal entry)
     auto product = [&](auto fin) {
         const int grp = lane >> lsh;
         const bool first = (lane & (L - 1)) == 0;
-        for (int s = wid; s < nsl; s += RWARPS) {
+        for (int s = wid, sn = 2 * RWARPS - 1 - wid; s < nsl; rs_next(s, sn)) {
             const int off = so[s], w = (so[s + 1] - off) >> 5;
             const int pos = s * (32 >> lsh) + grp;
             const int rl = (pos & ~(RS_WINDOW - 1)) + perm[pos];
@@ -152,7 +152,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     };
     unsigned long long epoch = 1;
     // r = b - A x, the Jacobi inverse (slot 0 of a row is its diagonal), z
-    for (int i = tid; i < nu; i += RT) halo[i] = __ldcg(xg + list[i]);
+    for (int i = tid; i < nu; i += RT) halo[rs_swz(i)] = __ldcg(xg + list[i]);
     __syncthreads();
     double part[4] = {0.0, 0.0, 0.0, 0.0};
     bool bad = false;
@@ -201,14 +201,14 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
             for (int k = 0; k < 2; ++k)
                 if (i0 + k * RT < nu) {
                     const double2 m = c_mul(be, o[k]);
-                    halo[i0 + k * RT] = make_double2(z[k].x + m.x, z[k].y + m.y);
+                    halo[rs_swz(i0 + k * RT)] = make_double2(z[k].x + m.x, z[k].y + m.y);
                 }
         }
         __syncthreads();
         part[0] = part[1] = part[2] = part[3] = 0.0;
         product([&](int rl, double2 qi, const double2 *) {
             q[rl] = qi;
-            const double2 pq = c_mul(pown[rl], qi);
+            const double2 pq = c_mul(halo[rs_swz(own + rl)], qi);
             part[0] += pq.x;
             part[1] += pq.y;
         });
@@ -229,7 +229,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
         const double2 al = st.alpha;
         part[0] = part[1] = part[2] = part[3] = 0.0;
         for (int i = tid; i < nloc; i += RT) {
-            const double2 pi = pown[i], dx = c_mul(al, pi), dr = c_mul(al, q[i]);
+            const double2 pi = halo[rs_swz(own + i)], dx = c_mul(al, pi), dr = c_mul(al, q[i]);
             double2 xi = x[i], ri = r[i];
             xi.x += dx.x;
             xi.y += dx.y;

@@ -45,6 +45,7 @@ constexpr int RS_WINDOW = 256;       // rows sorted by length together
 constexpr int RS_SMEM_MAX = 224 * 1024;
 constexpr size_t RS_MAX_WAVES = 4;   // launches of one batch
 constexpr int RS_HOLD = 150 * 1024;  // matrix bytes a block is meant to hold
+constexpr int64_t RS_DEAL_BYTES = 2 << 20;   // matrix bytes per block when blocks are dealt out
 constexpr int RS_COPIES = 8;         // copies of the partial sums, at most
 constexpr int RM = 6;                // rigid-body modes of a piece (cfem_coarse.cuh)
 
@@ -76,8 +77,14 @@ __host__ __device__ inline size_t rs_meta_bytes(int rows, int lsh) {
     const size_t nsl = (size_t)rs_slices(rows, lsh);
     return rs_al((nsl + 1) * 4) + rs_al(nsl << (5 - lsh));
 }
+// Place of a halo entry, its low five bits mixed with the next five. A slice's
+// lanes hold rows of one kind (sorted by length), whose k-th columns lie a
+// fixed stride apart, 8 on a Tet10 mesh: 8 of 32 lanes met in each of 4 banks
+// (a batch of 48 Tet10 meshes: 53.7 ms without, 49.2 with). Applied to the
+// local columns when they are made, and to the halo's and the own rows' places.
+__host__ __device__ inline int rs_swz(int i) { return i ^ ((i >> 5) & 31); }
 __host__ __device__ inline size_t rs_halo_bytes(int u, int bs, size_t ts) {
-    return rs_al((size_t)u * 4) + rs_al((size_t)u * bs * ts);
+    return rs_al((size_t)u * 4) + (size_t)((u + 31) & ~31) * bs * ts;
 }
 // ... of the coarse correction: the block's rows of the coarse inverse, the
 // sums of all pieces, the rows' coordinates in their piece.
@@ -221,6 +228,15 @@ template <> struct SlotGroup<double> {
     using V = double;
     using C = uint16_t;
 };
+// A warp's next slice: 2 RWARPS - 1 - w, 2 RWARPS + w, 4 RWARPS - 1 - w, ... after
+// its first, w. A window's slices go from its longest rows to its shortest, so
+// with equal steps the same warps had the longest ones each time (products of a
+// block of 332,000 entries 80 -> 62 us).
+__device__ __forceinline__ void rs_next(int &s, int &next) {
+    const int after = s + 2 * RWARPS;
+    s = next;
+    next = after;
+}
 // Slots per group of a slice's layout.
 __host__ __device__ inline int rs_group(int bs, size_t ts) { return bs == 1 && ts == 4 ? 4 : 1; }
 __device__ __forceinline__ int rs_slot(int k, int lane, int q) {
@@ -378,6 +394,53 @@ __device__ __forceinline__ void rs_row_dd3(const uint16_t *cp, const double *vp,
     }
 }
 
+// One lane's part of a CSR row for the FP64 true residual, entries k, k + LANES,
+// ... as acc_R, a few loaded together: one at a time, each waiting for its column
+// and then for x there, a residual of the Tet10 elastic box of 27 x 15 x 13 cells
+// took 125 us, now 85. x comes through L1: the grid's last sum ordered its writes
+// before these reads.
+template <bool INIT, int BS>
+__device__ __forceinline__ void rs_row_R(const SysDev &S, int32_t k, int32_t k1, int64_t row,
+                                         double acc[BS], double alo[BS], double aab[BS],
+                                         double accf[BS], double dg[BS * BS]) {
+    constexpr int U = BS == 1 ? 4 : 2, B2 = BS * BS;
+    const double *x = S.x;
+    for (; k < k1; k += U * LANES) {
+        int64_t j[U];
+        double a[U][B2], xj[U][BS];
+        bool fj[U][BS];
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = __ldg(S.ci + (k + u * LANES < k1 ? k + u * LANES : k));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const double *vk = S.v64 + (int64_t)(k + u * LANES < k1 ? k + u * LANES : k) * B2;
+#pragma unroll
+            for (int e = 0; e < B2; ++e) a[u][e] = __ldg(vk + e);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int d = 0; d < BS; ++d) {
+                xj[u][d] = x[j[u] * BS + d];
+                fj[u][d] = INIT && S.fixed ? __ldg(S.fixed + j[u] * BS + d) != 0 : false;
+            }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (k + u * LANES >= k1) break;
+#pragma unroll
+            for (int c = 0; c < BS; ++c)
+#pragma unroll
+                for (int d = 0; d < BS; ++d) {
+                    const double ax = a[u][c * BS + d] * xj[u][d];
+                    dd_fma(acc[c], alo[c], a[u][c * BS + d], xj[u][d]);
+                    aab[c] += fabs(ax);
+                    if (INIT && fj[u][d]) accf[c] += ax;
+                    if (INIT && j[u] == row) dg[c * BS + d] = a[u][c * BS + d];
+                }
+        }
+    }
+}
+
 // list: (system, its block) of every block of the launch. A launch runs its
 // systems to the end, or for max_iters iterations when they may go on in a
 // later launch (keep: the residual and the Jacobi inverse then stay in
@@ -426,7 +489,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     int32_t *list = (int32_t *)area;
     area += rs_al((size_t)nu * 4);
     T *halo = (T *)area;
-    area += rs_al((size_t)nu * BS * sizeof(T));
+    area += (size_t)((nu + 31) & ~31) * BS * sizeof(T);
     T *q, *r, *dinv;
     const uint8_t *fx;
     if (S.vsm) {
@@ -494,7 +557,8 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
         for (int i = tid; i < n16; i += RT) ((int4 *)mv)[i] = __ldcs((const int4 *)gv + i);
         for (int i = tid; i < eres / 8; i += RT) ((int4 *)mc)[i] = __ldcs((const int4 *)gc + i);
     }
-    const T *pown = halo + (size_t)sh.own * BS;  // the direction on the block's own rows
+    const int own = sh.own;                      // the direction on the block's own rows
+    auto hplace = [](int i) { return BS == 1 ? rs_swz(i) : 3 * rs_swz(i / 3) + i % 3; };
     __syncthreads();
 
     // the words of an earlier launch hold its epochs: go on from there
@@ -601,13 +665,13 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (i0 + k * RT < nh) halo[i0 + k * RT] = zeta * g[k].x + beta * g[k].y;
+                    if (i0 + k * RT < nh) halo[hplace(i0 + k * RT)] = zeta * g[k].x + beta * g[k].y;
             }
             __syncthreads();
             double pq = 0.0;
             const int grp = lane >> lsh;
             const bool first = (lane & (L - 1)) == 0;
-            for (int s = wid; s < nsl; s += RWARPS) {
+            for (int s = wid, sn = 2 * RWARPS - 1 - wid; s < nsl; rs_next(s, sn)) {
                 const int off = so[s], w = (so[s + 1] - off) >> 5;
                 const int pos = s * (32 >> lsh) + grp;
                 const int rl = (pos & ~(RS_WINDOW - 1)) + perm[pos];
@@ -616,13 +680,13 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                 T pi[BS], acc[BS];
 #pragma unroll
                 for (int c = 0; c < BS; ++c) {
-                    pi[c] = pown[ri * BS + c];
+                    pi[c] = halo[BS * rs_swz(own + ri) + c];
                     acc[c] = 0;
                 }
                 if constexpr (BS == 1) {
                     const int at = off + SlotGroup<T>::Q * lane;
                     acc[0] = s < nres ? rs_row1<T, DIFF, true, 8>(mc + at, mv + at, w, first, halo, pi[0])
-                                      : rs_row1<T, DIFF, false, sizeof(T) == 4 ? 16 : 8>(gc + at, gv + at, w, first, halo, pi[0]);
+                                      : rs_row1<T, DIFF, false, sizeof(T) == 4 ? 24 : 8>(gc + at, gv + at, w, first, halo, pi[0]);
                 } else {
                     if (s < nres)
                         rs_row3<T, DIFF, true>(mc + off + lane, mv + 9 * (size_t)off + lane, w, first,
@@ -662,24 +726,41 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
             const T alpha = (T)alpha64;
             double rz = 0.0, rr = 0.0;
             double *x = S.x + d0;
-            for (int i = tid; i < nd; i += RT) {
-                const bool fixed = fx && fx[i];
-                const T pi = pown[i];
-                T rv = r[i];
-                if (!fixed) {
-                    x[i] += alpha64 * (double)pi;
-                    rv -= alpha * q[i];
-                    r[i] = rv;
+            // (all loads of four rows first: one at a time, a block of 10,600
+            // rows with its vectors in global memory took 20 us, now 7)
+            for (int i0 = tid; i0 < nd; i0 += 4 * RT) {
+                double xv[4];
+                T pi[4], rv[4], qv[4], dv[4];
+                bool fixed[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = i0 + k * RT < nd ? i0 + k * RT : i0;
+                    fixed[k] = fx && fx[i];
+                    xv[k] = x[i];
+                    rv[k] = r[i];
+                    qv[k] = q[i];
+                    dv[k] = dinv[i];
+                    pi[k] = halo[hplace(BS * own + i)];
                 }
-                T zv = dinv[i] * rv;
-                if constexpr (CO) zv = (T)((double)zv + coarse_at(i / 3, i % 3));
-                if (fixed) zv = (T)0;
-                P2 g;
-                g.x = zv;
-                g.y = pi;
-                pair[d0 + i] = g;
-                rz += (double)rv * (double)zv;
-                rr += (double)rv * (double)rv;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int i = i0 + k * RT;
+                    if (i >= nd) break;
+                    if (!fixed[k]) {
+                        x[i] = xv[k] + alpha64 * (double)pi[k];
+                        rv[k] -= alpha * qv[k];
+                        r[i] = rv[k];
+                    }
+                    T zv = dv[k] * rv[k];
+                    if constexpr (CO) zv = (T)((double)zv + coarse_at(i / 3, i % 3));
+                    if (fixed[k]) zv = (T)0;
+                    P2 g;
+                    g.x = zv;
+                    g.y = pi[k];
+                    pair[d0 + i] = g;
+                    rz += (double)rv[k] * (double)zv;
+                    rr += (double)rv[k] * (double)rv[k];
+                }
             }
             part[0] = rz;
             part[1] = rr;
@@ -698,13 +779,13 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (i0 + k * RT < nh) hx[i0 + k * RT] = g[k];
+                    if (i0 + k * RT < nh) hx[hplace(i0 + k * RT)] = g[k];
             }
             __syncthreads();
             double rr = 0.0, rp = 0.0, rz = 0.0, aa = 0.0;
             const int grp = lane >> lsh;
             const bool first = (lane & (L - 1)) == 0;
-            for (int s = wid; s < nsl; s += RWARPS) {
+            for (int s = wid, sn = 2 * RWARPS - 1 - wid; s < nsl; rs_next(s, sn)) {
                 const int off = so[s], w = (so[s + 1] - off) >> 5;
                 const int pos = s * (32 >> lsh) + grp;
                 const int rl = (pos & ~(RS_WINDOW - 1)) + perm[pos];
@@ -768,23 +849,39 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
             const int sub = lane & (LANES - 1), grp = lane / LANES;
             double rr = 0.0, s1 = 0.0, rz = 0.0, aa = 0.0;
             bool bad = false;
+            // Scalar rows: a row's bounds are loaded a pass ahead, and what follows
+            // its sum before the sum (a time step of the 40 x 36 x 33 P1 box 190 -> 178
+            // us); 3x3 rows have no registers left
+            // for it (residuals of the Tet10 box of 27 x 15 x 13 cells 85 -> 125 us)
+            constexpr bool AHEAD = BS == 1;
+            int32_t kn = 0, kn1 = 0;
+            if (AHEAD && wid * RPP + grp < nloc) {
+                kn = __ldg(S.rp + r0 + wid * RPP + grp);
+                kn1 = __ldg(S.rp + r0 + wid * RPP + grp + 1);
+            }
             for (int base = wid * RPP; base < nloc; base += RWARPS * RPP) {
                 const int rl = base + grp;
                 const bool valid = rl < nloc;
                 const int64_t row = r0 + (valid ? rl : 0);
+                const int32_t k0 = AHEAD ? kn : __ldg(S.rp + row), k1 = AHEAD ? kn1 : __ldg(S.rp + row + 1);
+                if (AHEAD && rl + RWARPS * RPP < nloc) {
+                    kn = __ldg(S.rp + row + RWARPS * RPP);
+                    kn1 = __ldg(S.rp + row + RWARPS * RPP + 1);
+                }
+                double b1 = 0.0;
+                T py1 = (T)0;
+                if (AHEAD && valid && sub == 0) {
+                    b1 = __ldg(S.b + d0 + rl);
+                    if (!init) py1 = pair[d0 + rl].y;
+                }
                 double acc[BS], alo[BS], accf[BS], aab[BS], dg[B2];
 #pragma unroll
                 for (int c = 0; c < BS; ++c) acc[c] = alo[c] = accf[c] = aab[c] = 0.0;
 #pragma unroll
                 for (int c = 0; c < B2; ++c) dg[c] = 0.0;
                 if (valid) {
-                    const int32_t k1 = __ldg(S.rp + row + 1);
-                    if (init)
-                        for (int32_t k = __ldg(S.rp + row) + sub; k < k1; k += LANES)
-                            acc_R<true, BS>(S.v64, S.ci, k, row, S.x, S.fixed, acc, alo, aab, accf, dg);
-                    else
-                        for (int32_t k = __ldg(S.rp + row) + sub; k < k1; k += LANES)
-                            acc_R<false, BS>(S.v64, S.ci, k, row, S.x, S.fixed, acc, alo, aab, accf, dg);
+                    if (init) rs_row_R<true, BS>(S, k0 + sub, k1, row, acc, alo, aab, accf, dg);
+                    else rs_row_R<false, BS>(S, k0 + sub, k1, row, acc, alo, aab, accf, dg);
                 }
 #pragma unroll
                 for (int c = 0; c < BS; ++c) {
@@ -800,7 +897,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                     for (int c = 0; c < BS; ++c) {
                         const int i = rl * BS + c;
                         const bool fixed = fx && fx[i];
-                        const double bi = __ldg(S.b + d0 + i);
+                        const double bi = AHEAD ? b1 : __ldg(S.b + d0 + i);
                         const double rt = fixed ? 0.0 : dd_residual(bi, acc[c], alo[c]);
                         rr += rt * rt;
                         if (!fixed) aa += aab[c] * aab[c];
@@ -822,7 +919,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
                             dv = dinv[i];
                         }
                         P2 g;
-                        g.y = init ? (T)0 : pair[d0 + i].y;
+                        g.y = init ? (T)0 : (AHEAD ? py1 : pair[d0 + i].y);
                         if (!init) s1 += (double)rv * (double)g.y;
                         if (!CO) {
                             g.x = fixed ? (T)0 : dv * rv;
@@ -904,13 +1001,13 @@ __global__ void k_rs_split(const SysDev *__restrict__ sys, RsCta *ctas, int n, i
     if (i >= n) return;
     const SysDev &S = sys[ctas[i].sys];
     const int c = ctas[i].cta;
-    const int64_t total = __ldg(S.rp + S.n) + (int64_t)alpha * S.n;
+    const int64_t first = __ldg(S.rp), total = __ldg(S.rp + S.n) - first + (int64_t)alpha * S.n;
     auto bound = [&](int k) {   // first row with k / ncta of the work before it
         const int64_t want = total * k / S.ncta;
         int64_t lo = 0, hi = S.n;
         while (lo < hi) {
             const int64_t mid = (lo + hi) >> 1;
-            if (__ldg(S.rp + mid) + alpha * mid < want) lo = mid + 1; else hi = mid;
+            if (__ldg(S.rp + mid) - first + alpha * mid < want) lo = mid + 1; else hi = mid;
         }
         return (int32_t)lo;
     };
@@ -1021,11 +1118,11 @@ k_rs_cols(const SysDev *__restrict__ sys, const RsCta *__restrict__ ctas,
     __syncthreads();
     const int lsh = S.lsh, L = 1 << lsh, rs = 32 >> lsh, u = lane & (L - 1);
     auto place = [&](int32_t c) {
-        if ((uint32_t)c >= (uint32_t)S.n) return (uint16_t)0;   // not a column of this matrix
+        if ((uint32_t)c >= (uint32_t)S.n) return (uint16_t)rs_swz(0);   // not a column of this matrix
         const int w = c >> 5, g = w >> 2;
         int v = pre[g];
         for (int j = 4 * g; j < w; ++j) v += __popc(rs_bits[j]);
-        return (uint16_t)(v + __popc(rs_bits[w] & ((1u << (c & 31)) - 1u)));
+        return (uint16_t)rs_swz(v + __popc(rs_bits[w] & ((1u << (c & 31)) - 1u)));
     };
     const uint8_t *perm = S.sperm + me.sl0 * 32;
     for (int s = wid; s < rs_slices(me.rows, lsh); s += RWARPS) {
