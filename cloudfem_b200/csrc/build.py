@@ -17,7 +17,7 @@ OUT = os.path.join(os.path.dirname(HERE), "libcfem.so")
 SOURCES = ["cfem_core.cu", "cfem_pattern.cu", "cfem_assemble.cu",
            "cfem_dirichlet.cu", "cfem_solve.cu", "cfem_complex.cu", "cfem_em.cu",
            "cfem_faces.cu"]
-HEADERS = ["cfem_common.cuh", "cfem_coarse.cuh", "cfem_cocg.cuh", "cfem_resident.cuh", "cfem_tables.cuh"]
+HEADERS = ["cfem_common.cuh", "cfem_coarse.cuh", "cfem_order.cuh", "cfem_cocg.cuh", "cfem_resident.cuh", "cfem_tables.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr",
          "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

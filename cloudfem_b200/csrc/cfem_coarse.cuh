@@ -22,7 +22,7 @@
 // 17 x 14 in FP64 763 -> 176, 9.2 -> 5.0 ms. An iteration costs 15 us instead of
 // 10.7 on the first: the six sums and their way through memory.
 //
-// Set-up, in this file: Morton order and a copy of the system in it, the
+// Set-up, in this file: Morton order (cfem_order.cuh copies the system), the
 // pieces' geometry, P^T A P by blocks of 6 x 6, and its inverse.
 
 constexpr int RC_NB = 40;            // neighbour pieces accumulated at a time
@@ -72,7 +72,7 @@ __device__ __forceinline__ uint32_t rc_spread(uint32_t v) {   // 10 bits, two ze
 // Morton keys on a grid of cubic cells, 1024 along the longest edge.
 __global__ void k_rc_morton(const double *__restrict__ nodes, int64_t n,
                             const unsigned long long *__restrict__ lo,
-                            const unsigned long long *__restrict__ hi, uint32_t *__restrict__ key,
+                            const unsigned long long *__restrict__ hi, unsigned long long *__restrict__ key,
                             int32_t *__restrict__ id) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -89,51 +89,6 @@ __global__ void k_rc_morton(const double *__restrict__ nodes, int64_t n,
     }
     key[i] = k;
     id[i] = (int32_t)i;
-}
-
-// Inverse of the order, and the row lengths in it.
-__global__ void k_rc_rows(const int32_t *__restrict__ ord, const int32_t *__restrict__ rp, int64_t n,
-                          int32_t *__restrict__ inv, int32_t *__restrict__ len) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i > n) return;
-    if (i == n) {
-        len[n] = 0;
-        return;
-    }
-    const int32_t o = ord[i];
-    inv[o] = (int32_t)i;
-    len[i] = rp[o + 1] - rp[o];
-}
-// The system in the new order, one warp per block row.
-__global__ void __launch_bounds__(256)
-k_rc_permute(const SysDev S, const int32_t *__restrict__ ord, const int32_t *__restrict__ inv,
-             const int32_t *__restrict__ rpn, int32_t *__restrict__ ci, double *__restrict__ v64,
-             float *__restrict__ v32, double *__restrict__ b, double *__restrict__ x,
-             uint8_t *__restrict__ fixed) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < S.n; i += nw) {
-        const int64_t o = ord[i], k0 = S.rp[o], len = S.rp[o + 1] - k0, t0 = rpn[i];
-        for (int64_t k = lane; k < len; k += 32) {
-            const int32_t c = S.ci[k0 + k];
-            ci[t0 + k] = (uint32_t)c < (uint32_t)S.n ? inv[c] : (int32_t)i;
-        }
-        for (int64_t k = lane; k < 9 * len; k += 32) v64[9 * t0 + k] = S.v64[9 * k0 + k];
-        if (v32)
-            for (int64_t k = lane; k < 9 * len; k += 32) v32[9 * t0 + k] = S.v32[9 * k0 + k];
-        if (lane < 3) {
-            b[3 * i + lane] = S.b[3 * o + lane];
-            x[3 * i + lane] = S.x[3 * o + lane];
-            fixed[3 * i + lane] = S.fixed ? S.fixed[3 * o + lane] : 0;
-        }
-    }
-}
-__global__ void k_rc_back(const int32_t *__restrict__ ord, int64_t n, const double *__restrict__ xn,
-                          double *__restrict__ x) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= 3 * n) return;
-    const int64_t i = t / 3;
-    x[3 * (int64_t)ord[i] + (t - 3 * i)] = xn[t];
 }
 
 // Coordinates of every block's nodes from their mean, in units of the piece's

@@ -3021,6 +3021,7 @@ __global__ void k_loop_cond(cudaGraphConditionalHandle h, GridBar *bar, unsigned
 }
 #include "cfem_resident.cuh"
 #include "cfem_cocg.cuh"
+#include "cfem_order.cuh"
 #include "cfem_coarse.cuh"
 
 }  // namespace cfem
@@ -3157,6 +3158,20 @@ static int gxs_prepare() {
 // different host threads and overlap on the device). A solve resets the
 // solver state, runs k_pcg_init and then the persistent kernel or graph
 // replays until every system has finished.
+// Copy of systems in another row order (cfem_order.cuh); what it holds lives in
+// one allocation. The copies' row pointers count entries over all systems.
+struct RowOrder {
+    int ns = 0, bs = 1;
+    bool mixed = false;
+    int64_t rows = 0, entries = 0;
+    char *mem = nullptr;
+    cfem::OrderDev *src = nullptr;
+    int32_t *ord = nullptr, *inv = nullptr, *rp = nullptr, *ci = nullptr;
+    double *v64 = nullptr, *b = nullptr, *x = nullptr;
+    float *v32 = nullptr;
+    uint8_t *fixed = nullptr;
+};
+
 struct cfem_pcg_plan {
     cfem_ctx *ctx = nullptr;
     int device = 0;
@@ -3168,11 +3183,14 @@ struct cfem_pcg_plan {
     bool rs_dense = false;        // ... in the batch shape
     bool rs_keep = false;         // ... a solve slot: goes on over several launches
     bool rs_co = false;           // ... with the coarse correction
+    std::vector<int> rs_n;        // blocks of each system
+    RowOrder ro;                  // ... and the copy of the systems in another row order
+    bool rs_dealt = false;        // ... fewer than its entries ask for, to fit one launch
     std::vector<int2> waves;      // (first block, blocks) in the launch list
     int2 *rs_list = nullptr;      // launch list: (system, block)
     cfem::RsCta *d_ctas = nullptr;   // block table
     size_t rs_ts = 8;                // bytes of a vector entry (complex: 16)
-    int rs_ctas = 0, rs_smem = 0, rs_vsm = 0;
+    int rs_ctas = 0, rs_smem = 0;
     int2 *rs_ucnt = nullptr;         // every block's halo size and rows
     int32_t *rs_ulist = nullptr;     // every block's halo
     char *rs_col = nullptr, *rs_val = nullptr;
@@ -3472,6 +3490,7 @@ static void plan_free(cfem_pcg_plan *P) {
         if (P->ws_smeta) cudaFreeAsync(P->ws_smeta, P->w);
         if (P->tmpl_mem) cudaFreeAsync(P->tmpl_mem, P->w);
         if (P->ws_sdata) cudaFreeAsync(P->ws_sdata, P->w);
+        if (P->ro.mem) cudaFreeAsync(P->ro.mem, P->w);
         if (P->scan_tmp) cudaFreeAsync(P->scan_tmp, P->w);
         cudaStreamSynchronize(P->w);
     }
@@ -3492,8 +3511,127 @@ static void plan_free(cfem_pcg_plan *P) {
 }
 
 // ------------------------------------------------- resident scheduler, host
+// (Re)copies what the systems hold now, and the solution back.
+static dim3 order_grid(const RowOrder &R) {
+    return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(2048, 8192 / R.ns)), (unsigned)R.ns);
+}
+static int order_copy(const RowOrder &R, int what, cudaStream_t s) {
+    if (!R.mixed) what &= ~RO_V32;
+    if (R.bs == 3)
+        CFEM_LAUNCH(k_ro_copy<3>, order_grid(R), 256, 0, s, R.src, R.ord, R.inv, R.rp, R.ci, R.v64, R.v32,
+                    R.b, R.x, R.fixed, what);
+    else
+        CFEM_LAUNCH(k_ro_copy<1>, order_grid(R), 256, 0, s, R.src, R.ord, R.inv, R.rp, R.ci, R.v64, R.v32,
+                    R.b, R.x, R.fixed, what);
+    return CFEM_OK;
+}
+static int order_back(const RowOrder &R, cudaStream_t s) {
+    if (R.bs == 3) CFEM_LAUNCH(k_ro_back<3>, order_grid(R), 256, 0, s, R.src, R.ord, R.x);
+    else CFEM_LAUNCH(k_ro_back<1>, order_grid(R), 256, 0, s, R.src, R.ord, R.x);
+    return CFEM_OK;
+}
+// The order of d_nodes' Morton keys (one system), or by lowest column, and the
+// copy in it: its pattern, and `what`. On failure nothing is held.
+static int order_build(RowOrder &R, const cfem_linsys *L, const int32_t *nnzb, int ns,
+                       const double *d_nodes, int what, cudaStream_t s) {
+    R.ns = ns;
+    R.bs = L[0].bs;
+    R.mixed = L[0].mode == CFEM_SOLVE_MIXED;
+    std::vector<OrderDev> src(ns);
+    for (int i = 0; i < ns; ++i) {
+        src[i] = OrderDev{L[i].d_row_ptr, L[i].d_col, L[i].d_vals64, L[i].d_b, L[i].d_vals32,
+                          L[i].d_fixed, L[i].d_x, L[i].n_rows, R.rows};
+        R.rows += L[i].n_rows;
+        R.entries += nnzb[i];
+    }
+    const int64_t n = R.rows, e = R.entries, b2 = R.bs * R.bs;
+    CFEM_CHECK(n < INT32_MAX && e < INT32_MAX, CFEM_ERR_INVALID, "row order: too large");
+    int sys_bits = 0;
+    while ((1 << sys_bits) < ns) ++sys_bits;
+    const int end_bit = d_nodes ? 30 : 32 + sys_bits;
+    size_t scan_bytes = 0, sort_bytes = 0;
+    CFEM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const int32_t *)nullptr,
+                                            (int32_t *)nullptr, n + 1, s));
+    CFEM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const unsigned long long *)nullptr,
+                                              (unsigned long long *)nullptr, (const int32_t *)nullptr,
+                                              (int32_t *)nullptr, (int)n, 0, end_bit, s));
+    char *base = nullptr, *work = nullptr;
+    size_t off = 0;
+    auto take = [&](char *m, size_t b) { char *p = m ? m + off : nullptr; off += align256(b); return (void *)p; };
+    unsigned long long *box = nullptr, *key = nullptr, *key2 = nullptr;
+    int32_t *id = nullptr, *len = nullptr;
+    void *tmp = nullptr;
+    auto hold = [&]() {
+        off = 0;
+        R.src = (OrderDev *)take(base, ns * sizeof(OrderDev));
+        R.ord = (int32_t *)take(base, n * 4);
+        R.inv = (int32_t *)take(base, n * 4);
+        R.rp = (int32_t *)take(base, (n + 1) * 4);
+        R.ci = (int32_t *)take(base, e * 4);
+        R.v64 = (double *)take(base, e * b2 * 8);
+        R.v32 = R.mixed ? (float *)take(base, e * b2 * 4) : nullptr;
+        R.b = (double *)take(base, n * R.bs * 8);
+        R.x = (double *)take(base, n * R.bs * 8);
+        R.fixed = (uint8_t *)take(base, n * R.bs);
+    };
+    auto pass = [&]() {
+        off = 0;
+        box = (unsigned long long *)take(work, 6 * 8);
+        key = (unsigned long long *)take(work, n * 8);
+        key2 = (unsigned long long *)take(work, n * 8);
+        id = (int32_t *)take(work, n * 4);
+        len = (int32_t *)take(work, (n + 1) * 4);
+        tmp = take(work, std::max(scan_bytes, sort_bytes));
+    };
+    hold();
+    CFEM_TRY(tmp_alloc(&base, off, s));
+    R.mem = base;
+    hold();
+    auto run = [&]() -> int {
+        pass();
+        CFEM_TRY(tmp_alloc(&work, off, s));
+        pass();
+        CFEM_CUDA(cudaMemcpyAsync(R.src, src.data(), ns * sizeof(OrderDev), cudaMemcpyHostToDevice, s));
+        if (d_nodes) {
+            CFEM_CUDA(cudaMemsetAsync(box, 0xff, 3 * 8, s));
+            CFEM_CUDA(cudaMemsetAsync(box + 3, 0, 3 * 8, s));
+            CFEM_LAUNCH(k_rc_box, std::min(grid_for(n, 256), 64u), 256, 0, s, d_nodes, n, box, box + 3);
+            CFEM_LAUNCH(k_rc_morton, grid_for(n, 256), 256, 0, s, d_nodes, n, box, box + 3, key, id);
+        } else {
+            CFEM_LAUNCH(k_ro_mincol, dim3(64, (unsigned)ns), 256, 0, s, R.src, key, id);
+        }
+        CFEM_CUDA(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, key, key2, id, R.ord, (int)n, 0, end_bit, s));
+        CFEM_LAUNCH(k_ro_rows, grid_for(n + 1, 256), 256, 0, s, R.src, key2, R.ord, n, R.inv, len);
+        CFEM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, len, R.rp, n + 1, s));
+        return order_copy(R, RO_COLS | what, s);
+    };
+    const int st = run();
+    tmp_free(work, s);
+    if (st != CFEM_OK) {
+        tmp_free(R.mem, s);
+        R = RowOrder{};
+    }
+    return st;
+}
+// The copies as linear systems.
+static std::vector<cfem_linsys> order_systems(const RowOrder &R, const cfem_linsys *L) {
+    std::vector<cfem_linsys> M(L, L + R.ns);
+    int64_t base = 0;
+    for (cfem_linsys &m : M) {
+        m.d_row_ptr = R.rp + base;
+        m.d_col = R.ci;
+        m.d_vals64 = R.v64;
+        m.d_vals32 = R.v32;
+        m.d_b = R.b + base * R.bs;
+        m.d_x = R.x + base * R.bs;
+        m.d_fixed = R.fixed + base * R.bs;
+        base += m.n_rows;
+    }
+    return M;
+}
+
 // Shape of one system from its rows, stored blocks and block size alone (the
-// same alone and in a batch). A block takes at least about 2,560 stored
+// same alone and in a batch of a few launches). A block takes at least about 2,560 stored
 // entries (1,024 3x3 blocks): more blocks make the two grid-wide sums of an
 // iteration dearer (16 / 63 / 148 blocks: 4.4 / 5.4 / 6.9 us) than their
 // share of the products saves; a 20^3 P1 box ran 9.0, 7.8 and 9.4 us per
@@ -3508,17 +3646,16 @@ static void plan_free(cfem_pcg_plan *P) {
 // on the whole GPU (whose sums cost the same however little there is to add).
 // 24 served systems of 1,000 to 60,000 unknowns: 170 -> 38 ms against rounds of
 // captured launches over every slot's capacity.
-static void rs_shape(int64_t n, int64_t nnzb, int bs, size_t ts, bool dense, int num_sms, int &ncta,
-                     int &lsh) {
+static int rs_blocks(int64_t nnzb, int bs, size_t ts, bool dense, int num_sms) {
     const int64_t per = dense ? RS_HOLD / (int64_t)(2 + bs * bs * ts) : (bs == 3 ? 1024 : 2560);
-    ncta = (int)std::max<int64_t>(1, std::min<int64_t>((nnzb + per - 1) / per, num_sms));
+    return (int)std::max<int64_t>(1, std::min<int64_t>((nnzb + per - 1) / per, num_sms));
+}
+static int rs_lanes(int64_t n, int64_t nnzb, int bs, int ncta) {   // log2 of the lanes per row
     const int64_t mean = nnzb / n, rows = n / ncta;
-    if (bs == 3) {
-        lsh = mean >= 20 ? 2 : 1;
-    } else {
-        lsh = 0;
-        while (lsh < 3 && ((rows << lsh) >> 5) < 12 && (mean >> lsh) >= 16) ++lsh;
-    }
+    if (bs == 3) return mean >= 20 ? 2 : 1;
+    int lsh = 0;
+    while (lsh < 3 && ((rows << lsh) >> 5) < 12 && (mean >> lsh) >= 16) ++lsh;
+    return lsh;
 }
 
 // Work of a row beside its stored entries (k_rs_split), and with it the
@@ -3535,18 +3672,27 @@ static size_t rs_map_bytes(int64_t n, int64_t rows, int lsh) {
 // Whether the batch may run on the resident scheduler, and its launches:
 // every system of one precision and block size, point Jacobi, the set-up's
 // column bitmap within shared memory, as many whole systems to a launch as the
-// SMs hold blocks and at most RS_MAX_WAVES launches. A larger batch is the
-// graph scheduler's, whose launches share their latencies among all systems:
-// 48 Tet10 heat meshes of 4 to 24 cells (45 M entries) took 79 ms in the dense
-// shape, 64 ms with four times its entries per block, 58 ms as a graph.
+// SMs hold blocks and at most RS_MAX_WAVES launches. A larger batch, up to one
+// system per SM, takes one launch with the blocks dealt out by expected work,
+// entries times iterations (which grow as the cube root of the rows on a
+// mesh), over a copy of the systems in an order with compact blocks
+// (cfem_order.cuh): every system then runs from start to end beside the
+// others, each meeting only its own blocks. Its blocks stream matrices that
+// outgrow shared memory, so past RS_DEAL_BYTES per block it has no advantage
+// left over the graph scheduler's launches over all systems. Whole calls with
+// Tet10 heat meshes of a to b cells per edge, graph -> dealt: in mixed precision
+// 8 meshes of 20-24 39 -> 20 ms, 48 of 4-12 22 -> 7.6, 48 of 4-24 (1.8 MB per
+// block) 68 -> 48, 100 of 4-16 50 -> 39, 140 of 4-20 (4 MB) 106 -> 108; in
+// FP64 16 of 8-16 16 -> 12, 24 of 4-24 (1.5 MB) 44 -> 43, 100 of 4-16 48 -> 57.
+// (As whole systems in several launches the 48 took 64 ms.)
 static bool rs_plan(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t *nnzb) {
     const int sms = std::min(P->ctx->num_sms, RS_MAX_CTAS);
     const size_t ts = systems[0].mode == CFEM_SOLVE_MIXED ? 4 : P->rs_ts;
-    int used = 0, total = 0;
-    P->waves.clear();
-    for (int i = 0; i < P->n_systems; ++i) {
+    const int ns = P->n_systems, bs = systems[0].bs;
+    P->rs_n.clear();
+    for (int i = 0; i < ns; ++i) {
         const cfem_linsys &L = systems[i];
-        if (L.bs != systems[0].bs || L.mode != systems[0].mode || nnzb[i] <= 0 ||
+        if (L.bs != bs || L.mode != systems[0].mode || nnzb[i] <= 0 ||
             (L.bs == 3 && L.precond != CFEM_PRECOND_JACOBI))
             return false;
         // P1 elasticity in mixed precision keeps its former schedulers: at
@@ -3554,20 +3700,52 @@ static bool rs_plan(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
         // FP32 iteration (up to 1e-8 under thermal loads, any order of sums
         // another 1e-9), Tet10 elasticity's by 1e-10 and less
         if (L.bs == 3 && L.mode == CFEM_SOLVE_MIXED && nnzb[i] < 20 * L.n_rows) return false;
-        int ncta, lsh;
-        rs_shape(L.n_rows, nnzb[i], L.bs, ts, P->rs_dense, sms, ncta, lsh);
-        if (rs_map_bytes(L.n_rows, rs_most_rows(L.n_rows, nnzb[i], L.bs, ncta), lsh) >
-            (size_t)RS_SMEM_MAX)
-            return false;
-        if (P->waves.empty() || used + ncta > sms) {
-            P->waves.push_back(make_int2(total, 0));
-            used = 0;
-            if (P->waves.size() > RS_MAX_WAVES) return false;
-        }
-        used += ncta;
-        total += ncta;
-        P->waves.back().y += ncta;
+        P->rs_n.push_back(rs_blocks(nnzb[i], bs, ts, P->rs_dense, sms));
     }
+    auto pack = [&]() {                       // whole systems, in order, to launches
+        int used = 0, total = 0;
+        P->waves.clear();
+        for (int c : P->rs_n) {
+            if (P->waves.empty() || used + c > sms) {
+                P->waves.push_back(make_int2(total, 0));
+                used = 0;
+            }
+            used += c;
+            total += c;
+            P->waves.back().y += c;
+        }
+    };
+    pack();
+    // (PERSISTENT: as many launches as it takes, so that a system's answer does
+    // not depend on the others of its batch)
+    if (P->waves.size() > RS_MAX_WAVES && P->ctx->scheduler != CFEM_SCHED_PERSISTENT) {
+        int64_t entries = 0;
+        for (int i = 0; i < ns; ++i) entries += nnzb[i];
+        if (P->rs_dense || ns > sms || entries * (int64_t)(2 + bs * bs * ts) > RS_DEAL_BYTES * sms)
+            return false;
+        // one launch, the blocks dealt out one by one to the system whose
+        // blocks have the most to do
+        std::vector<double> work(ns);
+        for (int i = 0; i < ns; ++i) work[i] = (double)nnzb[i] * cbrt((double)systems[i].n_rows);
+        std::vector<int> most = P->rs_n;
+        P->rs_n.assign(ns, 1);
+        for (int left = sms - ns; left > 0; --left) {
+            int top = -1;
+            for (int i = 0; i < ns; ++i)
+                if (P->rs_n[i] < most[i] &&
+                    (top < 0 || work[i] * P->rs_n[top] > work[top] * P->rs_n[i]))
+                    top = i;
+            if (top < 0) break;
+            ++P->rs_n[top];
+        }
+        P->rs_dealt = true;
+        pack();
+    }
+    for (int i = 0; i < ns; ++i)
+        if (!P->rs_dealt &&
+            rs_map_bytes(systems[i].n_rows, rs_most_rows(systems[i].n_rows, nnzb[i], bs, P->rs_n[i]),
+                         rs_lanes(systems[i].n_rows, nnzb[i], bs, P->rs_n[i])) > (size_t)RS_SMEM_MAX)
+            return false;
     return true;
 }
 
@@ -3584,6 +3762,7 @@ static int rs_vals(cfem_pcg_plan *P, cudaStream_t s) {
 
 static int rs_copies(cfem_pcg_plan *P, cudaStream_t s) {
     const SysDev &S = P->hs[0];
+    if (P->rs_dealt) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_V32, s));
     if (P->rs_ts == 16) return rs_vals<double2, 1>(P, s);
     if (S.mode == CFEM_SOLVE_MIXED) return S.bs == 3 ? rs_vals<float, 3>(P, s) : rs_vals<float, 1>(P, s);
     return S.bs == 3 ? rs_vals<double, 3>(P, s) : rs_vals<double, 1>(P, s);
@@ -3614,7 +3793,7 @@ static int rs_alloc(cfem_pcg_plan *P, char **out, size_t bytes, cudaStream_t s) 
 static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t *nnzb,
                     cudaStream_t s) {
     cfem_ctx *ctx = P->ctx;
-    const int sms = std::min(ctx->num_sms, RS_MAX_CTAS), ns = P->n_systems;
+    const int ns = P->n_systems;
     const int bs = systems[0].bs, mode = systems[0].mode;
     if (mode == CFEM_SOLVE_MIXED) P->rs_ts = 4;
     const size_t ts = P->rs_ts;
@@ -3646,7 +3825,8 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
         S.max_stall = L.max_stall > 0 ? L.max_stall : MAX_STALL;
         S.hist_cap = L.d_history ? L.history_cap : 0;
         S.hist = L.d_history;
-        rs_shape(L.n_rows, nnzb[i], bs, ts, P->rs_dense, sms, S.ncta, S.lsh);
+        S.ncta = P->rs_n[i];
+        S.lsh = rs_lanes(L.n_rows, nnzb[i], bs, S.ncta);
         S.sl0 = nslices;
         nslices += (S.n >> (5 - S.lsh)) + S.ncta + 1;
         for (int c = 0; c < S.ncta; ++c) ctas.push_back(RsCta{i, c, 0, 0, 0});
@@ -3681,6 +3861,20 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     CFEM_CUDA(cudaMemsetAsync(sizes, 0, (nslices + 1) * sizeof(int64_t), s));
     CFEM_LAUNCH(k_rs_split, grid_for(P->rs_ctas, 128), 128, 0, s, P->d_sys, P->d_ctas, P->rs_ctas,
                 rs_alpha(bs));
+    if (P->rs_dealt) {   // blocks of many rows: the bound on them is too wide, read them
+        CFEM_CUDA(cudaMemcpyAsync(ctas.data(), P->d_ctas, ctas.size() * sizeof(RsCta),
+                                  cudaMemcpyDeviceToHost, s));
+        CFEM_CUDA(cudaStreamSynchronize(s));
+        map_bytes = 0;
+        for (const RsCta &c : ctas)
+            map_bytes = std::max(map_bytes, rs_map_bytes(hs[c.sys].n, c.rows, hs[c.sys].lsh));
+        if (map_bytes > (size_t)RS_SMEM_MAX) {
+            tmp_free(P->ws_copy, s);
+            P->ws_copy = nullptr;
+            hs.assign(ns, SysDev{});
+            return CFEM_OK;
+        }
+    }
     CFEM_CUDA(cudaFuncSetAttribute(k_rs_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
     CFEM_CUDA(cudaFuncSetAttribute(k_rs_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
     CFEM_LAUNCH(k_rs_rank, (unsigned)P->rs_ctas, RT, map_bytes, s, P->d_sys, P->d_ctas, sizes, P->rs_ucnt,
@@ -3697,27 +3891,27 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     CFEM_CUDA(cudaMemcpyAsync(&total, soff + nslices, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     CFEM_CUDA(cudaMemcpyAsync(ucnt.data(), P->rs_ucnt, ctas.size() * 8, cudaMemcpyDeviceToHost, s));
     CFEM_CUDA(cudaStreamSynchronize(s));
-    // shared memory of the largest block: its halo always, its vectors if
-    // every block of the batch has room for them
-    int umax = 0;
-    size_t meta = 0, vec = 0;
-    for (size_t c = 0; c < ctas.size(); ++c) {
-        umax = std::max(umax, ucnt[c].x);
-        meta = std::max(meta, rs_meta_bytes(ucnt[c].y, hs[ctas[c].sys].lsh));
-        vec = std::max(vec, rs_vec_bytes(ucnt[c].y, bs, ts));
-    }
-    // (with the coarse correction, 3 KB more of static shared memory)
+    // shared memory of a system's largest block: its halo always, its vectors
+    // if every block of the system has room for them (with the coarse
+    // correction, 3 KB more of static shared memory)
     const size_t smem_max = P->rs_co ? RS_SMEM_MAX - 4096 : RS_SMEM_MAX;
-    size_t fixed = meta + rs_halo_bytes(umax, bs, ts);
-    if (P->rs_co)
-        for (const int2 &u : ucnt) fixed = std::max(fixed, meta + rs_halo_bytes(umax, bs, ts) + rs_coarse_bytes(u.y, hs[0].ncta));
-    P->rs_vsm = fixed + vec <= smem_max;
-    if (P->rs_vsm) fixed += vec;
+    int umax = 0;
+    size_t fixed = 0;
     size_t state = align256(ns * sizeof(SysState)) + align256(sizeof(GridBar));
-    for (const SysDev &S : hs) {
+    for (size_t c = 0, i = 0; i < hs.size(); ++i) {
+        SysDev &S = hs[i];
+        size_t need = 0, vec = 0;
+        for (int k = 0; k < S.ncta; ++k, ++c) {
+            umax = std::max(umax, ucnt[c].x);
+            need = std::max(need, rs_meta_bytes(ucnt[c].y, S.lsh) + rs_halo_bytes(ucnt[c].x, bs, ts) +
+                                      (P->rs_co ? rs_coarse_bytes(ucnt[c].y, S.ncta) : 0));
+            vec = std::max(vec, rs_vec_bytes(ucnt[c].y, bs, ts));
+        }
+        S.vsm = need + vec <= smem_max;
+        fixed = std::max(fixed, need + (S.vsm ? vec : 0));
         const size_t nd = (size_t)S.n * bs;
         state += align256(nd * 2 * ts) + align256(rs_mail_bytes(S.ncta)) +
-                 (P->rs_vsm && !P->rs_keep ? 0 : 3 * align256(nd * ts));
+                 (S.vsm && !P->rs_keep ? 0 : 3 * align256(nd * ts));
     }
     // halo lists, as far apart as the system's longest
     size_t lists = 0;
@@ -3750,7 +3944,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     for (SysDev &S : hs) {
         const size_t nd = (size_t)S.n * bs;
         S.pair = take_s(nd * 2 * ts);
-        if (!P->rs_vsm || P->rs_keep) {
+        if (!S.vsm || P->rs_keep) {
             S.q = take_s(nd * ts);
             S.r = take_s(nd * ts);
             S.dinv = take_s(nd * ts);
@@ -3766,7 +3960,6 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
         S.ulist = P->rs_ulist + l0;
         S.rcol = (const uint16_t *)P->rs_col;
         S.rval = P->rs_val;
-        S.vsm = P->rs_vsm;
         c0 += S.ncta;
         l0 += (size_t)S.ncta * S.umax;
     }
@@ -3798,10 +3991,11 @@ static int rs_launch(cfem_pcg_plan *P, const SysDev *d_sys, SysState *d_st, Grid
 }
 
 static int rs_run(cfem_pcg_plan *P, cudaStream_t w) {
+    if (P->rs_dealt) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_VEC, w));   // read anew by each solve
     for (const int2 &v : P->waves)
         CFEM_TRY(rs_launch(P, P->d_sys, P->d_st, P->d_bar, P->rs_list + v.x, v.y, P->hs[0].bs,
                            P->hs[0].mode, P->rs_smem, 3 * P->max_iter + 16, INT32_MAX, w));
-    return CFEM_OK;
+    return P->rs_dealt ? order_back(P->ro, w) : CFEM_OK;
 }
 
 // COCG of one complex symmetric system on the resident layout (see
@@ -3920,8 +4114,18 @@ static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,
     if (!P->slots &&
         (ctx->scheduler == CFEM_SCHED_AUTO || ctx->scheduler == CFEM_SCHED_PERSISTENT) &&
         rs_plan(P, systems, nnzbs.data())) {
-        CFEM_TRY(rs_build(P, systems, nnzbs.data(), s));
+        int st = CFEM_OK;
+        std::vector<cfem_linsys> copies;
+        if (P->rs_dealt) {
+            st = order_build(P->ro, systems, nnzbs.data(), n_systems, nullptr, 0, s);
+            if (st == CFEM_OK) copies = order_systems(P->ro, systems);
+        }
+        if (st == CFEM_OK)
+            CFEM_TRY(rs_build(P, P->rs_dealt ? copies.data() : systems, nnzbs.data(), s));
         if (P->resident) return CFEM_OK;
+        tmp_free(P->ro.mem, s);           // does not fit: the graph scheduler
+        P->ro = RowOrder{};
+        P->rs_dealt = false;
     }
     size_t state_bytes = 0, copy_bytes = 0;
     for (int i = 0; i < n_systems; ++i) {
@@ -5130,45 +5334,18 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
     // 5.3 -> 3.5 and 13.5 -> 6.9 ms (whole FP64 calls)
     if (nnzb < 2048 || !rs_plan(&P, &L, &nnzb)) return CFEM_OK;
     const int64_t n = L.n_rows;
-    int ncta, lsh;
-    rs_shape(n, nnzb, 3, L.mode == CFEM_SOLVE_MIXED ? 4 : 8, false, std::min(ctx->num_sms, RS_MAX_CTAS),
-             ncta, lsh);
+    const int ncta = P.rs_n[0];
     const size_t nm = (size_t)RM * ncta;
     const bool mixed = L.mode == CFEM_SOLVE_MIXED;
-    size_t scan_bytes = 0, sort_bytes = 0;
-    CFEM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (const int32_t *)nullptr,
-                                            (int32_t *)nullptr, n + 1, s));
-    CFEM_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, (const uint32_t *)nullptr,
-                                              (uint32_t *)nullptr, (const int32_t *)nullptr,
-                                              (int32_t *)nullptr, (int)n, 0, 30, s));
     char *mem = nullptr;
     size_t off = 0;
     auto take = [&](size_t b) { char *p = mem ? mem + off : nullptr; off += align256(b); return (void *)p; };
-    unsigned long long *box = nullptr;
-    uint32_t *key = nullptr, *key2 = nullptr;
-    int32_t *id = nullptr, *ord = nullptr, *inv = nullptr, *len = nullptr, *rp = nullptr, *ci = nullptr;
-    double *v64 = nullptr, *b = nullptr, *x = nullptr, *ac = nullptr, *rowbuf = nullptr, *ainv = nullptr,
-           *gall = nullptr;
-    float *v32 = nullptr, *xl = nullptr;
-    uint8_t *fixed = nullptr, *own = nullptr;
+    double *ac = nullptr, *rowbuf = nullptr, *ainv = nullptr, *gall = nullptr;
+    float *xl = nullptr;
+    uint8_t *own = nullptr;
     unsigned *flag = nullptr;
-    void *tmp = nullptr;
     auto lay = [&]() {
         off = 0;
-        box = (unsigned long long *)take(6 * 8);
-        key = (uint32_t *)take(n * 4);
-        key2 = (uint32_t *)take(n * 4);
-        id = (int32_t *)take(n * 4);
-        ord = (int32_t *)take(n * 4);
-        inv = (int32_t *)take(n * 4);
-        len = (int32_t *)take((n + 1) * 4);
-        rp = (int32_t *)take((n + 1) * 4);
-        ci = (int32_t *)take((size_t)nnzb * 4);
-        v64 = (double *)take((size_t)nnzb * 72);
-        v32 = mixed ? (float *)take((size_t)nnzb * 36) : nullptr;
-        b = (double *)take(n * 24);
-        x = (double *)take(n * 24);
-        fixed = (uint8_t *)take(n * 3);
         own = (uint8_t *)take(n);
         xl = (float *)take(n * 12);
         ac = (double *)take(nm * nm * 8);
@@ -5176,7 +5353,6 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         ainv = (double *)take(nm * nm * 8);
         gall = (double *)take(nm * 8);
         flag = (unsigned *)take((size_t)RS_COPIES * ncta * 4);
-        tmp = take(std::max(scan_bytes, sort_bytes));
     };
     lay();
     CFEM_TRY(tmp_alloc(&mem, off, s));
@@ -5186,39 +5362,15 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         CFEM_CUDA(cudaEventCreate(&e0));
         CFEM_CUDA(cudaEventCreate(&e1));
         CFEM_CUDA(cudaEventRecord(e0, s));
-        CFEM_CUDA(cudaMemsetAsync(box, 0xff, 3 * 8, s));
-        CFEM_CUDA(cudaMemsetAsync(box + 3, 0, 3 * 8, s));
-        CFEM_LAUNCH(k_rc_box, std::min(grid_for(n, 256), 64u), 256, 0, s, d_nodes, n, box, box + 3);
-        CFEM_LAUNCH(k_rc_morton, grid_for(n, 256), 256, 0, s, d_nodes, n, box, box + 3, key, id);
-        CFEM_CUDA(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, key, key2, id, ord, (int)n, 0, 30, s));
-        CFEM_LAUNCH(k_rc_rows, grid_for(n + 1, 256), 256, 0, s, ord, L.d_row_ptr, n, inv, len);
-        CFEM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, len, rp, n + 1, s));
-        SysDev src{};
-        src.n = n;
-        src.rp = L.d_row_ptr;
-        src.ci = L.d_col;
-        src.v64 = L.d_vals64;
-        src.v32 = L.d_vals32;
-        src.b = L.d_b;
-        src.x = L.d_x;
-        src.fixed = L.d_fixed;
-        CFEM_LAUNCH(k_rc_permute, std::min(grid_for(n * 32, 256), (unsigned)ctx->num_sms * 16), 256, 0, s,
-                    src, ord, inv, rp, ci, v64, v32, b, x, fixed);
-        cfem_linsys M = L;
-        M.d_row_ptr = rp;
-        M.d_col = ci;
-        M.d_vals64 = v64;
-        M.d_vals32 = v32;
-        M.d_b = b;
-        M.d_x = x;
-        M.d_fixed = fixed;
+        CFEM_TRY(order_build(P.ro, &L, &nnzb, 1, d_nodes, RO_V64 | RO_V32 | RO_VEC, s));
+        const cfem_linsys M = order_systems(P.ro, &L)[0];
         P.hs[0].ainv = ainv;
         P.hs[0].gall = gall;
         P.hs[0].xl = xl;
         CFEM_TRY(rs_build(&P, &M, &nnzb, s));
         if (!P.resident) return CFEM_OK;
         CFEM_CUDA(cudaMemsetAsync(P.ws_state, 0, P.state_bytes, s));
-        CFEM_LAUNCH(k_rc_geo, (unsigned)ncta, 256, 0, s, P.d_ctas, d_nodes, ord, xl, own);
+        CFEM_LAUNCH(k_rc_geo, (unsigned)ncta, 256, 0, s, P.d_ctas, d_nodes, P.ro.ord, xl, own);
         CFEM_CUDA(cudaMemsetAsync(ac, 0, nm * nm * 8, s));
         CFEM_CUDA(cudaMemsetAsync(flag, 0, (size_t)RS_COPIES * ncta * 4, s));
         constexpr size_t acc_bytes = (size_t)RC_WARPS * RC_NB * 36 * 8;
@@ -5237,7 +5389,7 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         CFEM_CUDA(cudaEventRecord(e1, s));
         CFEM_TRY(noalloc_result(P.d_st, P.d_bar, stats, s));
         if (stats->status != CFEM_OK) return CFEM_OK;
-        CFEM_LAUNCH(k_rc_back, grid_for(3 * n, 256), 256, 0, s, ord, n, x, L.d_x);
+        CFEM_TRY(order_back(P.ro, s));
         float ms = 0.0f;
         CFEM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
         stats->kernel_ms = ms;
@@ -5247,7 +5399,7 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
     const int st = run();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    for (char *m : {P.ws_copy, P.ws_state, P.ws_sdata, mem}) tmp_free(m, s);
+    for (char *m : {P.ws_copy, P.ws_state, P.ws_sdata, P.ro.mem, mem}) tmp_free(m, s);
     return st;
 }
 }  // namespace cfem

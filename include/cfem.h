@@ -158,8 +158,11 @@ CFEM_API int cfem_ctx_destroy(cfem_ctx *ctx);
  *                 iterations, the host polling convergence once per replay
  *                 (every launch visible to per-launch profilers);
  * AUTO          - the resident kernel where it takes the systems in at most
- *                 four launches; else PERSISTENT when all row chunks fit in
- *                 one resident wave, else GRAPH (default). */
+ *                 four launches, or in one with fewer blocks per system (up
+ *                 to one system per SM and 2 MB of matrix per SM; a system's
+ *                 blocks, and the last bits of its answer, then depend on
+ *                 the batch); else PERSISTENT when all row chunks fit in one
+ *                 resident wave, else GRAPH (default). */
 enum { CFEM_SCHED_AUTO = 0, CFEM_SCHED_PERSISTENT = 1, CFEM_SCHED_GRAPH = 2,
        CFEM_SCHED_GRAPH_POLLED = 3 };
 CFEM_API int cfem_ctx_set_scheduler(cfem_ctx *ctx, int scheduler);
@@ -451,10 +454,12 @@ CFEM_API int cfem_mixed_matrix_batch(cfem_ctx *ctx, const cfem_mixed_job *jobs,
 /* ---- solver -------------------------------------------------------------
  * Jacobi-preconditioned CG on a batch of independent systems. A few systems
  * of one kind run on the resident kernel (whole solves in cooperative
- * launches, two grid-wide sums per iteration); larger batches are one graph
+ * launches, two grid-wide sums per iteration), and so do many small ones, each
+ * on its share of the SMs; larger batches are one graph
  * of per-phase launches (direction update, SpMV, reduction, update,
  * reduction per iteration). Per-system scalars are reduced in a fixed order, so each
- * result is bitwise the same alone and in any batch on a given scheduler.
+ * result is bitwise the same alone and in any batch on a given scheduler
+ * (PERSISTENT: any batch of systems of its kind; AUTO chooses by the batch).
  * CFEM_SOLVE_MIXED runs the CG in FP32 and keeps FP64 for the true residual
  * r = b - A x, the solution update and the convergence test (reliable
  * updates). Replaces spla.spsolve / spla.factorized (tet_poisson.py:121,

@@ -138,6 +138,72 @@ def test_batch_of_several_launches_equals_alone(torch, bs):
             assert torch.equal(alone.x, s.x)
 
 
+@pytest.mark.parametrize("bs", [1, 3])
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind,sizes", [
+    ("wide", [40, 500, 3000, 9000] * 12),       # more blocks than four launches hold
+    ("wide", [2000] * 148),                     # one block each on 148 SMs
+    ("wide", [2000] * 149),                     # ... one system too many
+    ("scatter", [60000] * 6 + [9000] * 24),     # columns that do not fit a block: not dealt
+])
+def test_batch_with_dealt_blocks(torch, kind, sizes, mode, bs):
+    """A batch in one launch with the blocks dealt out, over copies of the
+    systems in another row order: against the graph scheduler, then again
+    after the values, loads and Dirichlet data changed (a plan's second
+    solve must take all of them anew)."""
+    from cloudfem_b200 import _native as N
+    from cloudfem_b200.device import PcgPlan
+    if bs == 3:
+        sizes = [max(1, n // 3) for n in sizes]
+    rt = N.runtime()
+    md, rtol, tol = ((N.SOLVE_FP64, 1e-13, 1e-12) if mode == "fp64" else (N.SOLVE_MIXED, 1e-10, 1e-9))
+    made = {}
+    for n in set(sizes):
+        rng = np.random.default_rng(n)
+        A, blocks, cols, indptr, b, fixed, xd = _system(n, bs, kind, n)
+        # the rows in a random order, as a mesh generator may number its nodes
+        p = rng.permutation(n)
+        P = sp.csr_matrix((np.arange(len(cols)) + 1, cols, indptr), shape=(n, n))[p][:, p].tocsr()
+        dofs = (bs * p[:, None] + np.arange(bs)).ravel()
+        made[n] = (None, blocks[P.data - 1], P.indices.astype(np.int32), P.indptr.astype(np.int32),
+                   b[dofs], fixed[dofs], xd[dofs])
+    out = []
+    for sched in (N.SCHED_AUTO, N.SCHED_GRAPH):
+        N.check(rt.lib.cfem_ctx_set_scheduler(rt.ctx, sched))
+        try:
+            systems = [_block_system(torch, rt, made[n], bs) for n in sizes]
+            if md == N.SOLVE_MIXED:
+                for s in systems:
+                    s.ensure_fp32()
+            plan = PcgPlan(systems, md, rtol, 2000)
+            x0 = [s.x.clone() for s in systems]
+            got = []
+            for turn in range(2):
+                for s, x in zip(systems, x0):
+                    if turn:
+                        s.vals64.mul_(2.0)
+                        if s.vals32 is not None:
+                            s.vals32.mul_(2.0)
+                        s.b.mul_(-4.0)
+                    s.x.copy_(x * (-2.0 if turn else 1.0))
+                if turn:
+                    plan.refresh()
+                for r in plan.solve():
+                    assert r.status == N.CFEM_OK, r
+                got.append([s.x.cpu().numpy() for s in systems])
+            plan.close()
+        finally:
+            N.check(rt.lib.cfem_ctx_set_scheduler(rt.ctx, N.SCHED_AUTO))
+        out.append(got)
+    for turn in range(2):
+        for n, x, ref in zip(sizes, out[0][turn], out[1][turn]):
+            fixed, xd = made[n][5], made[n][6]
+            assert np.array_equal(x[fixed], xd[fixed] * (-2.0 if turn else 1.0))
+            assert np.linalg.norm(x - ref) <= 2 * tol * np.linalg.norm(ref)
+    for n, x, x2 in zip(sizes, out[0][0], out[0][1]):   # twice the matrix, -4 times the rest
+        assert np.linalg.norm(x2 + 2 * x) <= 4 * tol * np.linalg.norm(x)
+
+
 def test_refresh_takes_new_values(torch):
     from cloudfem_b200 import _native as N
     from cloudfem_b200.device import PcgPlan
