@@ -17,9 +17,9 @@
 // replacement computes them anew.
 //
 // Measured, iterations and time of a whole solve call, plain -> with it: Tet10
-// cantilever of 40 x 5 x 5 cells in FP64 1,740 -> 191, 23.7 -> 5.2 ms; Tet10 box
-// of 27 x 15 x 13 in mixed precision 1,814 -> 268, 39 -> 13.1 ms; P1 box of 31 x
-// 17 x 14 in FP64 763 -> 176, 9.2 -> 5.0 ms. An iteration costs 15 us instead of
+// cantilever of 40 x 5 x 5 cells in FP64 1,740 -> 191, 23.7 -> 5.0 ms; Tet10 box
+// of 27 x 15 x 13 in mixed precision 1,814 -> 268, 39 -> 11.0 ms; P1 box of 31 x
+// 17 x 14 in FP64 763 -> 176, 9.2 -> 4.8 ms. An iteration costs 15 us instead of
 // 10.7 on the first: the six sums and their way through memory.
 //
 // Set-up, in this file: Morton order (cfem_order.cuh copies the system), the
@@ -149,10 +149,15 @@ __device__ __forceinline__ void rc_mode(int p, double x, double y, double z, dou
     m[2] = p == 2 ? 1.0 : (p == 3 ? y : (p == 4 ? -x : 0.0));
 }
 
-// The block row of P^T A P that belongs to piece blockIdx.x. A warp walks its
-// rows' entries one at a time, its lanes holding the 36 values of a 6 x 6
-// block (the last four lanes two each), into accumulators of its own; the
-// warps' sums are added in warp order, so the result is the same every time.
+// The block row of P^T A P that belongs to piece blockIdx.x. A warp takes its
+// rows' entries 32 at a time: each lane fetches one entry's column, piece and
+// coordinates, then 18 lanes (d, q) go through the entries together and sum
+// T[d][q] = (A_ij C_j)[d][q], C_j the column node's modes, as long as the piece
+// stays the same (mostly: a row's columns are near it). R_i^T T, R_i the row
+// node's modes, goes into the warp's own sums for that piece, which are added
+// in warp order at the end, so the result is the same every time. (One entry
+// after the other, each waiting for its column, piece and coordinates: 1,320 us
+// on the Tet10 box of 27 x 15 x 13 cells, now 440.)
 constexpr int RC_WARPS = 16;
 __global__ void __launch_bounds__(32 * RC_WARPS)
 k_rc_ac(const SysDev *__restrict__ sys, const float *__restrict__ xl, const uint8_t *__restrict__ own,
@@ -180,6 +185,7 @@ k_rc_ac(const SysDev *__restrict__ sys, const float *__restrict__ xl, const uint
     __syncthreads();
     const int p0 = lane / 6, q0 = lane % 6, p1 = (lane + 32) / 6, q1 = (lane + 32) % 6;
     const bool two = lane < 4;                            // values lane and lane + 32
+    const int d = lane < 18 ? lane / 6 : 0;               // T[d][q0]
     for (int first = 0; first < count; first += RC_NB) {
         const int nb = min(RC_NB, count - first);
         double *acc = rc_acc + (size_t)w * RC_NB * 36;
@@ -187,35 +193,55 @@ k_rc_ac(const SysDev *__restrict__ sys, const float *__restrict__ xl, const uint
         __syncwarp();
         for (int i = w; i < me.rows; i += RC_WARPS) {
             const int64_t row = (int64_t)me.row0 + i;
-            double rp0[3], rp1[3];
+            double r0[3], r1[3];
             const float *xi = xl + 3 * row;
-            rc_mode(p0, xi[0], xi[1], xi[2], rp0);
-            rc_mode(two ? p1 : 0, xi[0], xi[1], xi[2], rp1);
+            rc_mode(p0, xi[0], xi[1], xi[2], r0);
+            rc_mode(two ? p1 : 0, xi[0], xi[1], xi[2], r1);
 #pragma unroll
-            for (int d = 0; d < 3; ++d)
-                if (S.fixed && __ldg(S.fixed + 3 * row + d)) rp0[d] = rp1[d] = 0.0;
-            const int32_t k1 = __ldg(S.rp + row + 1);
-            for (int32_t k = __ldg(S.rp + row); k < k1; ++k) {
-                const int64_t j = __ldg(S.ci + k);
-                const int b = slot[__ldg(own + j)] - first;
-                if (b < 0 || b >= nb) continue;           // uniform over the warp
-                const float *xj = xl + 3 * j;
-                const double x = xj[0], y = xj[1], z = xj[2];
-                double a[9], c0[3], c1[3];
-#pragma unroll
-                for (int e = 0; e < 9; ++e) a[e] = __ldg(S.v64 + 9 * (int64_t)k + e);
-                rc_mode(q0, x, y, z, c0);
-                rc_mode(two ? q1 : 0, x, y, z, c1);
+            for (int c = 0; c < 3; ++c)
+                if (S.fixed && __ldg(S.fixed + 3 * row + c)) r0[c] = r1[c] = 0.0;
+            const int32_t kb = __ldg(S.rp + row), ke = __ldg(S.rp + row + 1);
+            double T = 0.0;
+            int cur = -1;
+            auto flush = [&]() {                          // acc[cur] += R^T T
                 double s0 = 0.0, s1 = 0.0;
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    if (S.fixed && __ldg(S.fixed + 3 * j + d)) continue;
-                    s0 += (rp0[0] * a[d] + rp0[1] * a[3 + d] + rp0[2] * a[6 + d]) * c0[d];
-                    s1 += (rp1[0] * a[d] + rp1[1] * a[3 + d] + rp1[2] * a[6 + d]) * c1[d];
+                for (int c = 0; c < 3; ++c) {
+                    s0 += r0[c] * __shfl_sync(0xffffffffu, T, 6 * c + q0);
+                    s1 += r1[c] * __shfl_sync(0xffffffffu, T, 6 * c + q1);
                 }
-                acc[b * 36 + lane] += s0;
-                if (two) acc[b * 36 + 32 + lane] += s1;
+                if (cur >= 0) {
+                    acc[cur * 36 + lane] += s0;
+                    if (two) acc[cur * 36 + 32 + lane] += s1;
+                }
+                T = 0.0;
+            };
+            for (int32_t k0 = kb; k0 < ke; k0 += 32) {
+                const int32_t k = k0 + lane < ke ? k0 + lane : ke - 1;
+                const int64_t j = __ldg(S.ci + k);
+                const int bl = slot[__ldg(own + j)] - first;
+                const float x = __ldg(xl + 3 * j), y = __ldg(xl + 3 * j + 1), z = __ldg(xl + 3 * j + 2);
+                int fl = 0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) fl |= S.fixed && __ldg(S.fixed + 3 * j + c) ? 1 << c : 0;
+                const int m = min(32, ke - k0);
+#pragma unroll 4
+                for (int e = 0; e < m; ++e) {
+                    const int b = __shfl_sync(0xffffffffu, bl, e), f = __shfl_sync(0xffffffffu, fl, e);
+                    const float xe = __shfl_sync(0xffffffffu, x, e), ye = __shfl_sync(0xffffffffu, y, e),
+                                ze = __shfl_sync(0xffffffffu, z, e);
+                    const double *v = S.v64 + 9 * (int64_t)(k0 + e) + 3 * d;
+                    const double a0 = __ldg(v), a1 = __ldg(v + 1), a2 = __ldg(v + 2);
+                    if (b != cur) {                       // uniform over the warp
+                        flush();
+                        cur = b >= 0 && b < nb ? b : -1;
+                    }
+                    double c[3];
+                    rc_mode(q0, xe, ye, ze, c);
+                    T += a0 * (f & 1 ? 0.0 : c[0]) + a1 * (f & 2 ? 0.0 : c[1]) + a2 * (f & 4 ? 0.0 : c[2]);
+                }
             }
+            flush();
         }
         __syncthreads();
         for (int i = t; i < nb * 36; i += 32 * RC_WARPS) {
@@ -229,80 +255,107 @@ k_rc_ac(const SysDev *__restrict__ sys, const float *__restrict__ xl, const uint
 }
 
 // Inverse of the SPD matrix ac (nm x nm) by block Gauss-Jordan without
-// pivoting, block k the six rows of piece k held by its block in shared
-// memory. Step k needs only row block k: its owner scales and publishes it
-// with a flag, the others wait for the flag, read it and update their rows. A
-// pivot that has all but vanished (a mode that others span: a piece of
-// nodes on a line, or all its DOFs fixed) leaves its unknown out: zero row and
-// column. Waits are bounded; on expiry *err is set and every block returns.
+// pivoting, pivot blocks of RC_RB rows, each held by one block in shared memory
+// (the last padded with zero rows to nmp = nb RC_RB). Step k needs only the rows
+// of block k: their owner scales and publishes them with a flag, the others
+// wait for the flag, read them and update theirs; the next owner's first warp
+// meanwhile inverts its pivot block. A pivot that has all but vanished (a mode
+// that others span: a piece of nodes on a line, all its DOFs fixed, padding)
+// leaves its unknown out: zero row and column. A chain of nb steps of a few us,
+// mostly the way of flag and rows through L2: 148 pieces took 820 us with a
+// pivot block per piece, 690 with two. Waits are bounded; on expiry *err is
+// set and every block returns.
+constexpr int RC_RB = 2 * RM;
 __global__ void __launch_bounds__(RT, 1)
-k_rc_inv(const double *__restrict__ ac, int nblk, double *rowbuf, unsigned *flag, double *__restrict__ out,
-         int *err, unsigned long long timeout_ns) {
+k_rc_inv(const double *__restrict__ ac, int nm, int nb, double *rowbuf, unsigned *flag,
+         double *__restrict__ out, int *err, unsigned long long timeout_ns) {
     extern __shared__ __align__(16) double rc_rows[];     // the block's own rows
-    __shared__ double D[RM][RM], F[RM][RM], d0[RM];
+    __shared__ double D[RC_RB][RC_RB], d0[RC_RB];
+    __shared__ __align__(16) double Dt[RC_RB][RC_RB], Ft[RC_RB][RC_RB];   // [column][row]
     __shared__ int quit;
-    const int t = threadIdx.x, lane = t & 31, me = blockIdx.x, nm = RM * nblk;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5, me = blockIdx.x, nmp = RC_RB * nb;
     double *mine = rc_rows;
-    for (int i = t; i < RM * nm; i += RT) mine[i] = ac[(size_t)RM * me * nm + i];
+    for (int i = t; i < RC_RB * nmp; i += RT) {
+        const int r = RC_RB * me + i / nmp, c = i % nmp;
+        mine[i] = r < nm && c < nm ? ac[(size_t)r * nm + c] : 0.0;
+    }
     if (t == 0) quit = 0;
     __syncthreads();
-    if (t < RM) d0[t] = mine[t * nm + RM * me + t];
+    if (t < RC_RB) d0[t] = mine[t * nmp + RC_RB * me + t];
     __syncthreads();
-    for (int k = 0; k < nblk; ++k) {
-        if (k == me) {
-            if (t < 32) {                                  // D^-1, entries lane and lane + 32
-                for (int e = lane; e < RM * RM; e += 32) D[e / RM][e % RM] = mine[(e / RM) * nm + RM * k + e % RM];
-                __syncwarp();
-                for (int p = 0; p < RM; ++p) {
-                    const double d = D[p][p];
-                    const bool take = d > 1e-10 * d0[p] && d0[p] > 0.0;
-                    const double iv = take ? 1.0 / d : 0.0;
-                    double v[2];
+    // first warp: D = D^-1 in place, and Dt; lane (i, h) holds half h of row i
+    auto invert = [&]() {
+        constexpr int H = RC_RB / 2;
+        const int i = lane % RC_RB, h = lane / RC_RB;
+        double a[H];
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const int e = lane + 32 * u;
-                        if (e >= RM * RM) continue;
-                        const int i = e / RM, j = e % RM;
-                        if (i == p && j == p) v[u] = iv;
-                        else if (i == p) v[u] = D[p][j] * iv;
-                        else if (j == p) v[u] = -D[i][p] * iv;
-                        else v[u] = D[i][j] - D[i][p] * D[p][j] * iv;
-                    }
-                    __syncwarp();
+        for (int c = 0; c < H; ++c) a[c] = h < 2 ? D[i][H * h + c] : 0.0;
 #pragma unroll
-                    for (int u = 0; u < 2; ++u)
-                        if (lane + 32 * u < RM * RM) D[(lane + 32 * u) / RM][(lane + 32 * u) % RM] = v[u];
-                    __syncwarp();
-                }
+        for (int p = 0; p < RC_RB; ++p) {
+            double r[H];
+#pragma unroll
+            for (int c = 0; c < H; ++c) r[c] = __shfl_sync(0xffffffffu, a[c], p + RC_RB * min(h, 1));
+            const double f = __shfl_sync(0xffffffffu, a[p % H], i + RC_RB * (p / H));
+            const double dp = __shfl_sync(0xffffffffu, a[p % H], p + RC_RB * (p / H));
+            const bool take = dp > 1e-10 * d0[p] && d0[p] > 0.0;
+            const double iv = take ? 1.0 / dp : 0.0, g = i == p ? iv : -f * iv;
+#pragma unroll
+            for (int c = 0; c < H; ++c) a[c] = i == p ? r[c] * iv : a[c] + r[c] * g;
+            if (h == p / H) a[p % H] = g;
+        }
+        if (h < 2)
+#pragma unroll
+            for (int c = 0; c < H; ++c) {
+                D[i][H * h + c] = a[c];
+                Dt[H * h + c][i] = a[c];
             }
-            __syncthreads();
-            for (int j = t; j < nm; j += RT) {
-                double c[RM], r[RM];
+    };
+    // v[i] += M[p][i] x[p] over p: M's column by column from shared memory, all
+    // rows' sums side by side
+    auto times = [&](const double (*M)[RC_RB], const double x[RC_RB], double v[RC_RB]) {
+        asm volatile("" ::: "memory");    // (M again for each column: it would not fit registers)
 #pragma unroll
-                for (int i = 0; i < RM; ++i) c[i] = mine[i * nm + j];
+        for (int p = 0; p < RC_RB; ++p)
 #pragma unroll
-                for (int i = 0; i < RM; ++i) {
-                    r[i] = 0.0;
+            for (int i = 0; i < RC_RB; i += 2) {
+                const double2 m = *(const double2 *)&M[p][i];
+                v[i] += m.x * x[p];
+                v[i + 1] += m.y * x[p];
+            }
+    };
+    if (me == 0 && wid == 0) {
+        for (int e = lane; e < RC_RB * RC_RB; e += 32) D[e / RC_RB][e % RC_RB] = mine[(e / RC_RB) * nmp + e % RC_RB];
+        __syncwarp();
+        invert();
+    }
+    __syncthreads();
+    for (int k = 0; k < nb; ++k) {
+        if (k == me) {
+            for (int j = t; j < nmp; j += RT) {
+                double c[RC_RB], v[RC_RB];
 #pragma unroll
-                    for (int p = 0; p < RM; ++p) r[i] += D[i][p] * c[p];
+                for (int p = 0; p < RC_RB; ++p) {
+                    c[p] = mine[p * nmp + j];
+                    v[p] = 0.0;
                 }
-                const bool diag = j / RM == k;
+                times(Dt, c, v);
+                const bool diag = j / RC_RB == k;
 #pragma unroll
-                for (int i = 0; i < RM; ++i) {
-                    const double v = diag ? D[i][j - RM * k] : r[i];
-                    mine[i * nm + j] = v;
-                    rowbuf[(size_t)(RM * k + i) * nm + j] = v;
+                for (int i = 0; i < RC_RB; ++i) {
+                    if (diag) v[i] = D[i][j - RC_RB * k];
+                    mine[i * nmp + j] = v[i];
+                    rowbuf[(size_t)(RC_RB * k + i) * nmp + j] = v[i];
                 }
             }
             __syncthreads();
             if (t == 0) {
                 fence_gpu();
                 for (int c = 0; c < RS_COPIES; ++c)
-                    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flag + c * nblk + k), "r"(1u) : "memory");
+                    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(flag + c * nb + k), "r"(1u) : "memory");
             }
         } else {
             if (t == 0) {
-                const unsigned *f = flag + (me % RS_COPIES) * nblk + k;
+                const unsigned *f = flag + (me % RS_COPIES) * nb + k;
                 unsigned long long t0 = 0;
                 for (unsigned spin = 0; ld_acquire(f) == 0; ++spin)
                     if ((spin & 63u) == 63u) {
@@ -315,24 +368,44 @@ k_rc_inv(const double *__restrict__ ac, int nblk, double *rowbuf, unsigned *flag
                         }
                     }
             }
-            if (t >= 32 && t < 32 + RM * RM) F[(t - 32) / RM][(t - 32) % RM] = mine[((t - 32) / RM) * nm + RM * k + (t - 32) % RM];
+            for (int e = t - 32; e >= 0 && e < RC_RB * RC_RB; e += RT)
+                Ft[e % RC_RB][e / RC_RB] = -mine[(e / RC_RB) * nmp + RC_RB * k + e % RC_RB];
+            const bool next = k + 1 == me;
+            if (next && wid == RWARPS - 1)                // the next pivot block, as it is now
+                for (int e = lane; e < RC_RB * RC_RB; e += 32)
+                    D[e / RC_RB][e % RC_RB] = mine[(e / RC_RB) * nmp + RC_RB * me + e % RC_RB];
             __syncthreads();
             if (quit) return;
-            for (int j = t; j < nm; j += RT) {
-                double r[RM];
+            const double *rk = rowbuf + (size_t)RC_RB * k * nmp;
+            if (next && wid == 0) {
+                for (int e = lane; e < RC_RB * RC_RB; e += 32) {
+                    const int i = e / RC_RB, j = e % RC_RB;
+                    double v = D[i][j];
 #pragma unroll
-                for (int p = 0; p < RM; ++p) r[p] = __ldcg(rowbuf + (size_t)(RM * k + p) * nm + j);
-                const bool diag = j / RM == k;
-#pragma unroll
-                for (int i = 0; i < RM; ++i) {
-                    double v = diag ? 0.0 : mine[i * nm + j];
-#pragma unroll
-                    for (int p = 0; p < RM; ++p) v -= F[i][p] * r[p];
-                    mine[i * nm + j] = v;
+                    for (int p = 0; p < RC_RB; ++p) v += Ft[p][i] * __ldcg(rk + (size_t)p * nmp + RC_RB * me + j);
+                    D[i][j] = v;
                 }
+                __syncwarp();
+                invert();
+            }
+            const int lo = next ? 32 : 0;                 // threads that update
+            for (int j = t - lo; j >= 0 && j < nmp; j += RT - lo) {
+                double r[RC_RB], v[RC_RB];
+                const bool diag = j / RC_RB == k;
+#pragma unroll
+                for (int p = 0; p < RC_RB; ++p) {
+                    r[p] = __ldcg(rk + (size_t)p * nmp + j);
+                    v[p] = diag ? 0.0 : mine[p * nmp + j];
+                }
+                times(Ft, r, v);
+#pragma unroll
+                for (int i = 0; i < RC_RB; ++i) mine[i * nmp + j] = v[i];
             }
             __syncthreads();
         }
     }
-    for (int i = t; i < RM * nm; i += RT) out[(size_t)RM * me * nm + i] = mine[i];
+    for (int i = t; i < RC_RB * nmp; i += RT) {
+        const int r = RC_RB * me + i / nmp, c = i % nmp;
+        if (r < nm && c < nm) out[(size_t)r * nm + c] = mine[i];
+    }
 }

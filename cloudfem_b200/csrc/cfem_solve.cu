@@ -5336,6 +5336,7 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
     const int64_t n = L.n_rows;
     const int ncta = P.rs_n[0];
     const size_t nm = (size_t)RM * ncta;
+    int nb = (ncta * RM + RC_RB - 1) / RC_RB, inm = (int)nm;   // pivot blocks, unknowns
     const bool mixed = L.mode == CFEM_SOLVE_MIXED;
     char *mem = nullptr;
     size_t off = 0;
@@ -5349,10 +5350,10 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         own = (uint8_t *)take(n);
         xl = (float *)take(n * 12);
         ac = (double *)take(nm * nm * 8);
-        rowbuf = (double *)take(nm * nm * 8);
+        rowbuf = (double *)take((size_t)RC_RB * nb * RC_RB * nb * 8);
         ainv = (double *)take(nm * nm * 8);
         gall = (double *)take(nm * 8);
-        flag = (unsigned *)take((size_t)RS_COPIES * ncta * 4);
+        flag = (unsigned *)take((size_t)RS_COPIES * nb * 4);
     };
     lay();
     CFEM_TRY(tmp_alloc(&mem, off, s));
@@ -5372,17 +5373,17 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         CFEM_CUDA(cudaMemsetAsync(P.ws_state, 0, P.state_bytes, s));
         CFEM_LAUNCH(k_rc_geo, (unsigned)ncta, 256, 0, s, P.d_ctas, d_nodes, P.ro.ord, xl, own);
         CFEM_CUDA(cudaMemsetAsync(ac, 0, nm * nm * 8, s));
-        CFEM_CUDA(cudaMemsetAsync(flag, 0, (size_t)RS_COPIES * ncta * 4, s));
+        CFEM_CUDA(cudaMemsetAsync(flag, 0, (size_t)RS_COPIES * nb * 4, s));
         constexpr size_t acc_bytes = (size_t)RC_WARPS * RC_NB * 36 * 8;
         CFEM_CUDA(cudaFuncSetAttribute(k_rc_ac, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)acc_bytes));
         CFEM_LAUNCH(k_rc_ac, (unsigned)ncta, 32 * RC_WARPS, acc_bytes, s, P.d_sys, xl, own, ac);
-        const size_t inv_bytes = RM * nm * 8;
-        CFEM_CUDA(cudaFuncSetAttribute(k_rc_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
-        int nblk = ncta, *err = &P.d_bar->err;
+        const size_t inv_bytes = (size_t)RC_RB * RC_RB * nb * 8;
+        CFEM_CUDA(cudaFuncSetAttribute(k_rc_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX - 4096));
+        int *err = &P.d_bar->err;
         unsigned long long limit = P.bar_timeout_ns;
-        void *args[] = {(void *)&ac, (void *)&nblk, (void *)&rowbuf, (void *)&flag,
+        void *args[] = {(void *)&ac, (void *)&inm, (void *)&nb, (void *)&rowbuf, (void *)&flag,
                         (void *)&ainv, (void *)&err, (void *)&limit};
-        CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_rc_inv, dim3((unsigned)ncta), dim3(RT), args,
+        CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_rc_inv, dim3((unsigned)nb), dim3(RT), args,
                                               inv_bytes, s));
         g_launches.fetch_add(1, std::memory_order_relaxed);
         CFEM_TRY(rs_run(&P, s));
