@@ -359,6 +359,8 @@ def run_ours(args, rank, world, local_rank):
     kname, kprof = _block_spmv_kernel(rt, args.precision)
     traffic = (_profiled_traffic(kprof, "fp32" if args.precision == "mixed" else "fp64")
                if kprof else None)
+    if not spmv_ms:      # no SpMV launch of its own: the whole solve is one kernel
+        kname, traffic = "k_resident", None
     h2d = mesh.nodes.size * 8 + mesh.elements.size * 4
     d2h = 3 * mesh.n_nodes * 8
     value = world * free * args.steps / (ms * 1e-3)

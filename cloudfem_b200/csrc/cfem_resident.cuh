@@ -32,12 +32,13 @@
 // (0.6 halo, 1.8 products, 3.2 sum, 0.4 update, 4.3 sum); Tet10 box of 27 x
 // 15 x 13 cells, elasticity in FP32, 52 MB of blocks of which 60 % fit, 32
 // -> 19 us; Tet10 heat of 44,415 rows in FP32 45 -> 10.0 us; P1 heat of
-// 699,273 rows in FP64 (104 MB streamed per iteration at 5.2 TB/s) 60 -> 43 us.
+// 699,273 rows in FP64 (104 MB streamed per iteration) 60 -> 40 us.
 //
-// Sums depend on the system's own shape (block count, lanes per row), never
-// on what else is in the batch. There are two shapes, one for solves and a
-// denser one for solve slots (rs_shape); within either a result is bitwise the
-// same alone and in any batch.
+// Sums depend on the system's own block count and lanes per row. There are
+// two block counts, one for solves and a smaller one for solve slots
+// (rs_blocks), which depend on the system alone: within either a result is
+// bitwise the same alone and in any batch. Only a batch with dealt blocks
+// (rs_plan) has others.
 
 constexpr int RT = 512;              // threads per block
 constexpr int RWARPS = RT / 32;
