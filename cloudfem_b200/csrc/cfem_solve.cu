@@ -4632,6 +4632,19 @@ static int plan_run(cfem_pcg_plan *P, cfem_solve_stats *stats, cudaStream_t s) {
     return CFEM_OK;
 }
 
+// What was queued on s for the plan (its set-up, a refresh) comes before what
+// the plan's own stream does next, solves from any stream and the release of
+// its memory. Waits for s instead where the plan has no event yet.
+static int plan_follow(cfem_pcg_plan *P, cudaStream_t s) {
+    if (!P->w || !P->ev[0]) {
+        CFEM_CUDA(cudaStreamSynchronize(s));
+        return CFEM_OK;
+    }
+    CFEM_CUDA(cudaEventRecord(P->ev[0], s));
+    CFEM_CUDA(cudaStreamWaitEvent(P->w, P->ev[0], 0));
+    return CFEM_OK;
+}
+
 }  // namespace cfem
 
 extern "C" int cfem_pcg_plan_create(cfem_ctx *ctx, const cfem_linsys *systems,
@@ -4643,7 +4656,9 @@ extern "C" int cfem_pcg_plan_create(cfem_ctx *ctx, const cfem_linsys *systems,
     *out = nullptr;
     CFEM_TRY(set_device(ctx->device));
     cfem_pcg_plan *P = new cfem_pcg_plan();
-    const int st = plan_build(ctx, systems, n_systems, (cudaStream_t)stream, P);
+    int st = plan_build(ctx, systems, n_systems, (cudaStream_t)stream, P);
+    const int order = plan_follow(P, (cudaStream_t)stream);
+    if (st == CFEM_OK) st = order;
     if (st != CFEM_OK) {
         plan_free(P);
         return st;
@@ -4657,7 +4672,9 @@ extern "C" int cfem_pcg_plan_refresh(cfem_pcg_plan *plan, void *stream) {
     CFEM_API_BEGIN
     CFEM_CHECK(plan, CFEM_ERR_INVALID, "cfem_pcg_plan_refresh: plan is NULL");
     CFEM_TRY(set_device(plan->device));
-    return plan_copies(plan, (cudaStream_t)stream);
+    const int st = plan_copies(plan, (cudaStream_t)stream);
+    const int order = plan_follow(plan, (cudaStream_t)stream);
+    return st != CFEM_OK ? st : order;
     CFEM_API_END
 }
 
