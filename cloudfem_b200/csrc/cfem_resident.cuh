@@ -283,14 +283,23 @@ __device__ __forceinline__ void rs_load(const uint16_t *cp, const T *vp, int g, 
 // of the row in lane k % L); the row's slot 0 (diag: this lane holds it) is
 // the diagonal, or the row sum of the FP32 difference form (DIFF), whose
 // other slots multiply p_j - p_i. cp, vp: the lane's first group; w: slots.
+//
+// FP32 slots are loaded 24 at a time of a streaming slice and 8 of a held one,
+// and which slices are held depends on what else is in the launch. The sums must
+// not: slot e of every group has a running sum of its own, which takes the
+// groups in their order however many were loaded together (groups past the
+// last add zero). FP64 slots are loaded 8 at a time either way, and every load
+// has its own sum.
 template <typename T, bool DIFF, bool SM, int U>
-__device__ __forceinline__ T rs_groups1(const uint16_t *cp, const T *vp, int g, int n, bool diag,
-                                        const T *halo, T pi) {
+__device__ __forceinline__ void rs_groups1(const uint16_t *cp, const T *vp, int g, int n, bool diag,
+                                           const T *halo, T pi, T acc[SlotGroup<T>::Q]) {
     constexpr int Q = SlotGroup<T>::Q;
     typename SlotGroup<T>::C c[U];
     typename SlotGroup<T>::V a[U];
     rs_load<T, U, SM>(cp, vp, g, n, c, a);
-    T acc = 0;
+    T sum[Q];
+#pragma unroll
+    for (int e = 0; e < Q; ++e) sum[e] = Q == 1 ? (T)0 : acc[e];
 #pragma unroll
     for (int j = 0; j < U; ++j) {
         int cj[Q];
@@ -301,21 +310,23 @@ __device__ __forceinline__ T rs_groups1(const uint16_t *cp, const T *vp, int g, 
         for (int e = 0; e < Q; ++e) {
             T pj = halo[cj[e]];
             if (DIFF) pj = (diag && g + j == 0 && e == 0) ? pi : pj - pi;
-            acc += (g + j < n ? aj[e] : (T)0) * pj;
+            sum[e] += (g + j < n ? aj[e] : (T)0) * pj;
         }
     }
-    return acc;
+#pragma unroll
+    for (int e = 0; e < Q; ++e) acc[e] = Q == 1 ? acc[e] + sum[e] : sum[e];
 }
 template <typename T, bool DIFF, bool SM, int SLOTS>
 __device__ __forceinline__ T rs_row1(const uint16_t *cp, const T *vp, int w, bool diag,
                                      const T *halo, T pi) {
     constexpr int Q = SlotGroup<T>::Q, U = SLOTS / Q;
     const int n = w / Q;
-    T acc = 0;
+    T acc[Q] = {};
     int g = 0;
-    for (; n - g > U / 2; g += U) acc += rs_groups1<T, DIFF, SM, U>(cp, vp, g, n, diag, halo, pi);
-    if (g < n) acc += rs_groups1<T, DIFF, SM, U / 2>(cp, vp, g, n, diag, halo, pi);
-    return acc;
+    for (; n - g > U / 2; g += U) rs_groups1<T, DIFF, SM, U>(cp, vp, g, n, diag, halo, pi, acc);
+    if (g < n) rs_groups1<T, DIFF, SM, U / 2>(cp, vp, g, n, diag, halo, pi, acc);
+    if constexpr (Q == 4) return (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    else return acc[0];
 }
 
 // The same over 3x3 blocks: nine value planes of 32 lanes per step.
