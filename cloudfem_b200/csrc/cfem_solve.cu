@@ -3256,10 +3256,10 @@ struct cfem_pcg_plan {
     // slots on the resident kernel: each slot's system has a resident plan of
     // its own (`sub`), all advanced by one launch per round over `rs_list`
     std::vector<cfem_pcg_plan *> sub;
-    std::vector<char> rs_busy;        // the slot holds a resident system to advance
-    bool rs_dirty = true;             // rs_list is not that of rs_busy
-    int graph_busy = 0;               // slots whose systems run on the graphs
-    std::vector<char> on_graph;
+    enum { SLOT_EMPTY, SLOT_GRAPH, SLOT_RESIDENT };
+    std::vector<char> where;          // what runs, or ran, the slot's last system
+    std::vector<char> live;           // ... which is not known to have ended
+    bool rs_dirty = true;             // rs_list is not that of the live resident systems
     char *rs_mem = nullptr;           // system table, states, barrier word, launch list
     cfem::SysDev *rs_sys = nullptr;
     cfem::SysState *rs_st = nullptr;
@@ -4829,8 +4829,8 @@ extern "C" int cfem_pcg_slots_create(cfem_ctx *ctx, int32_t n_slots, int32_t bs,
         P->rs_bar = (GridBar *)(P->rs_mem + o_bar);
         P->rs_list = (int2 *)(P->rs_mem + o_list);
         P->sub.assign(n_slots, nullptr);
-        P->rs_busy.assign(n_slots, 0);
-        P->on_graph.assign(n_slots, 0);
+        P->where.assign(n_slots, cfem_pcg_plan::SLOT_EMPTY);
+        P->live.assign(n_slots, 0);
     }
     if (st == CFEM_OK) {
         P->tmpl = P->hs;
@@ -4851,6 +4851,21 @@ extern "C" int cfem_pcg_slots_create(cfem_ctx *ctx, int32_t n_slots, int32_t bs,
     *out = P;
     return CFEM_OK;
     CFEM_API_END
+}
+
+// The slot's system has ended, or gives way to another: no round advances it
+// again (a launch over graph slots runs through all slots' capacity).
+static void slot_ended(cfem_pcg_plan *P, int slot) {
+    P->live[slot] = 0;
+    P->rs_dirty = true;
+}
+static void slot_holds(cfem_pcg_plan *P, int slot, int where) {
+    slot_ended(P, slot);
+    P->where[slot] = (char)where;
+    P->live[slot] = 1;
+}
+static bool slot_runs(const cfem_pcg_plan *P, int slot, int where) {
+    return P->live[slot] && P->where[slot] == where;
 }
 
 // Puts a system into a slot on the resident kernel: a resident plan of its
@@ -4888,8 +4903,7 @@ static int rs_assign(cfem_pcg_plan *P, int slot, const cfem_linsys *L, int32_t n
     }
     rs_slot_free(P->sub[slot], w);    // after the rounds that read it
     P->sub[slot] = sub;
-    P->rs_busy[slot] = 1;
-    P->rs_dirty = true;
+    slot_holds(P, slot, cfem_pcg_plan::SLOT_RESIDENT);
     *taken = true;
     return CFEM_OK;
 }
@@ -4902,7 +4916,7 @@ static int rs_round(cfem_pcg_plan *P, int iters, cudaStream_t w) {
         P->waves.clear();
         int smem = 0;
         for (int i = 0; i < P->n_systems; ++i) {
-            if (!P->rs_busy[i]) continue;
+            if (!slot_runs(P, i, cfem_pcg_plan::SLOT_RESIDENT)) continue;
             const int n = P->sub[i]->hs[0].ncta;
             if (P->waves.empty() || P->waves.back().y + n > std::min(P->ctx->num_sms, RS_MAX_CTAS))
                 P->waves.push_back(make_int2((int)list.size(), 0));
@@ -4985,19 +4999,12 @@ extern "C" int cfem_pcg_slots_assign(cfem_pcg_plan *P, int32_t slot, const cfem_
     CFEM_CHECK(!sell3 || *P->h_total <= P->cap_sell[slot], CFEM_ERR_INVALID,
                "system's sliced-ELL layout has %lld blocks, slot %d holds %lld",
                (long long)*P->h_total, slot, (long long)P->cap_sell[slot]);
-    if (P->on_graph[slot]) {          // the slot's last system, if the graphs had it
-        P->on_graph[slot] = 0;
-        --P->graph_busy;
-    }
     if (T.bs == 1 || sell3) {
         bool taken = false;
         CFEM_TRY(rs_assign(P, slot, L, nnzb, s, &taken));
         if (taken) return CFEM_OK;
     }
-    P->rs_busy[slot] = 0;
-    P->rs_dirty = true;
-    P->on_graph[slot] = 1;
-    ++P->graph_busy;
+    slot_holds(P, slot, cfem_pcg_plan::SLOT_GRAPH);
     SysDev S = T;   // the slot's workspace, lists and copies
     if (sell3) {
         S.sperm = P->smeta[2 * slot + set].perm;
@@ -5053,7 +5060,9 @@ extern "C" int cfem_pcg_slots_run(cfem_pcg_plan *P, int32_t rounds, void *stream
     CFEM_CUDA(cudaEventRecord(P->ev[0], s));
     CFEM_CUDA(cudaStreamWaitEvent(w, P->ev[0], 0));
     CFEM_TRY(rs_round(P, POLL_ITERS * rounds, w));
-    for (int r = 0; r < rounds && P->graph_busy > 0; ++r) {
+    bool graphs = false;
+    for (int i = 0; i < P->n_systems; ++i) graphs |= slot_runs(P, i, cfem_pcg_plan::SLOT_GRAPH);
+    for (int r = 0; r < rounds && graphs; ++r) {
         CFEM_CUDA(cudaGraphLaunch(P->pexec[r & 1], w));
         g_launches.fetch_add((int64_t)P->per_iter * POLL_ITERS, std::memory_order_relaxed);
     }
@@ -5090,11 +5099,8 @@ extern "C" int cfem_pcg_slots_poll(cfem_pcg_plan *P, cfem_solve_stats *stats) {
     const int h_err = P->h_flags[3];
     for (int i = 0; i < n; ++i) {
         cfem_solve_stats &o = stats[i];
-        const SysState *hst = P->sub[i] && !P->on_graph[i] ? P->h_st + n : P->h_st;
-        if (P->rs_busy[i] && hst[i].phase == PH_DONE) {
-            P->rs_busy[i] = 0;
-            P->rs_dirty = true;
-        }
+        const SysState *hst = P->where[i] == cfem_pcg_plan::SLOT_RESIDENT ? P->h_st + n : P->h_st;
+        if (P->live[i] && hst[i].phase == PH_DONE) slot_ended(P, i);
         memset(&o, 0, sizeof(o));
         o.status = hst[i].phase == PH_DONE ? hst[i].status : CFEM_SLOT_RUNNING;
         o.iterations = hst[i].iter;
@@ -5118,8 +5124,7 @@ extern "C" int cfem_pcg_slots_release(cfem_pcg_plan *P, int32_t slot, void *stre
     cudaStream_t s = (cudaStream_t)stream, w = P->w;
     CFEM_CUDA(cudaEventRecord(P->ev[0], s));
     CFEM_CUDA(cudaStreamWaitEvent(w, P->ev[0], 0));
-    P->rs_busy[slot] = 0;
-    P->rs_dirty = true;
+    slot_ended(P, slot);
     CFEM_LAUNCH(k_slot_cancel, 1, 32, 0, w, P->rs_st + slot, P->rs_bar);
     CFEM_LAUNCH(k_slot_cancel, 1, 32, 0, w, P->d_st + slot, P->d_bar);
     CFEM_CUDA(cudaEventRecord(P->ev[1], w));
