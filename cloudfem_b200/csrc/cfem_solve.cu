@@ -4854,10 +4854,13 @@ extern "C" int cfem_pcg_slots_create(cfem_ctx *ctx, int32_t n_slots, int32_t bs,
 }
 
 // The slot's system has ended, or gives way to another: no round advances it
-// again (a launch over graph slots runs through all slots' capacity).
+// again (a launch over graph slots runs through all slots' capacity), and what
+// it had on the resident kernel goes back to the pool after the queued rounds.
 static void slot_ended(cfem_pcg_plan *P, int slot) {
     P->live[slot] = 0;
     P->rs_dirty = true;
+    rs_slot_free(P->sub[slot], P->w);
+    P->sub[slot] = nullptr;
 }
 static void slot_holds(cfem_pcg_plan *P, int slot, int where) {
     slot_ended(P, slot);
@@ -4901,9 +4904,8 @@ static int rs_assign(cfem_pcg_plan *P, int slot, const cfem_linsys *L, int32_t n
         rs_slot_free(sub, s);
         return st;
     }
-    rs_slot_free(P->sub[slot], w);    // after the rounds that read it
-    P->sub[slot] = sub;
     slot_holds(P, slot, cfem_pcg_plan::SLOT_RESIDENT);
+    P->sub[slot] = sub;
     *taken = true;
     return CFEM_OK;
 }

@@ -70,3 +70,50 @@ def test_graph_rounds_stop_with_their_last_system(torch, bs):
     eng.assign(_block_system(torch, rt, band, bs), 1e-10, 2000, tag="band")
     assert launches(1) == 1                          # the resident kernel alone
     eng.close()
+
+
+@pytest.mark.parametrize("ending", ["finished", "released"])
+def test_slots_give_their_memory_back(torch, ending):
+    """What a slot holds on the resident kernel (38 bytes a block of an FP32 3x3
+    system, 26 MB for each of these) is the pool's again once its system has
+    finished or was released, not when the slot is taken next."""
+    from cloudfem_b200 import _native as N
+    rt = N.runtime()
+    n, held = 30000, 4 * 20 * 2 ** 20
+    data = _system(n, 3, "wide", 1)
+    from cloudfem_b200.device import SlotEngine
+    eng = SlotEngine(rt, 4, 3, N.SOLVE_MIXED, n, 30 * n)
+    idle = rt.trim(0)
+    slots = [eng.assign(_block_system(torch, rt, data, 3), 1e-10, 2000, tag=i) for i in range(4)]
+    eng.run(1)
+    assert rt.trim(0) >= idle + held             # the measure sees them
+    if ending == "finished":
+        _rounds(eng, range(4))
+    else:
+        for s in slots:
+            eng.release(s)
+    assert rt.trim(0) <= idle + held // 4
+    eng.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_admission_estimates_cover_a_request(torch, precision):
+    """What the server takes off its budget for a request covers what the
+    request holds on the device while it is in a slot, the resident copy too."""
+    from cloudfem_b200 import _native as N
+    from cloudfem_b200 import serve
+    from cloudfem_b200.mesh import box_mesh, box_mesh_tet10
+    rt = N.runtime()
+    for kind, mesh in (("p1_heat", box_mesh(60, 60, 60)), ("t10_heat", box_mesh_tet10(24, 24, 24)),
+                       ("t10_elast", box_mesh_tet10(16, 16, 16))):
+        r = serve.Request(0, kind, mesh)
+        srv = serve.Server(precision=precision)
+        eng = srv._engine(kind, srv._slot_class(r))
+        torch.cuda.empty_cache()
+        before = rt.trim(0) + torch.cuda.memory_allocated()
+        slot = eng.assign(srv._system(r), srv.rtol, tag=r)
+        eng.run(1)
+        taken = rt.trim(0) + torch.cuda.memory_allocated() - before
+        assert 0 < taken <= r.bytes_estimate() + 64 * 2 ** 20, (kind, taken, r.bytes_estimate())
+        eng.release(slot)
+        eng.close()
