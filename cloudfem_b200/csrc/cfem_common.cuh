@@ -85,6 +85,7 @@ struct cfem_ctx {
                                        // entry-major copy (0)
     int barrier_timeout_us = 4000000;  // persistent grid-barrier wait limit
     int barrier_hold = 0;              // phantom barrier arrivals (fault injection)
+    int alloc_fail = 0;                // resident set-up: this allocation fails (fault injection)
     cudaStream_t work = nullptr;       // capture stream of the graph scheduler
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t tev[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // SpMV timing

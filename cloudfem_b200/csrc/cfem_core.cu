@@ -251,6 +251,11 @@ int cfem_ctx_set_param(cfem_ctx *ctx, int param, int value) {
                        "phantom barrier arrivals must be 0 or 1 (got %d)", value);
             ctx->barrier_hold = value;
             return CFEM_OK;
+        case CFEM_PARAM_ALLOC_FAIL:
+            CFEM_CHECK(value >= 0 && value <= 16, CFEM_ERR_INVALID,
+                       "failing allocation must be 0 (none) or 1 .. 16 (got %d)", value);
+            ctx->alloc_fail = value;
+            return CFEM_OK;
         default:
             return fail(CFEM_ERR_INVALID, "unknown parameter %d", param);
     }
@@ -270,6 +275,7 @@ int cfem_ctx_get_param(const cfem_ctx *ctx, int param) {
         case CFEM_PARAM_SLOT_SELL3: return ctx->slot_sell3;
         case CFEM_PARAM_BARRIER_TIMEOUT_US: return ctx->barrier_timeout_us;
         case CFEM_PARAM_BARRIER_HOLD: return ctx->barrier_hold;
+        case CFEM_PARAM_ALLOC_FAIL: return ctx->alloc_fail;
         default: return -1;
     }
 }

@@ -3201,6 +3201,7 @@ struct cfem_pcg_plan {
     char *rs_col = nullptr, *rs_val = nullptr;
     char *arena = nullptr;           // resident set-up without allocations: memory from here
     size_t arena_bytes = 0, arena_used = 0;
+    int rs_allocs = 0;               // allocations of the resident set-up so far
     int grid = 1;
     unsigned long long bar_timeout_ns = 4000000000ull;   // grid-barrier wait limit
     unsigned bar_hold = 0;                               // phantom arrivals (tests)
@@ -3510,6 +3511,24 @@ static void plan_free(cfem_pcg_plan *P) {
 }
 
 // ------------------------------------------------- resident scheduler, host
+// Memory of a resident plan: from the library's pool, or from the plan's
+// arena. *out null when there is none: the solve then goes where it would
+// have gone without the resident kernel, in that path's memory.
+// CFEM_PARAM_ALLOC_FAIL: the plan's n-th such allocation finds none.
+static int rs_alloc(cfem_pcg_plan *P, char **out, size_t bytes, cudaStream_t s) {
+    *out = nullptr;
+    if (++P->rs_allocs == P->ctx->alloc_fail) return CFEM_OK;
+    if (!P->arena) {
+        const int st = tmp_alloc(out, bytes, s);
+        if (st == CFEM_ERR_NOMEM) (void)cudaGetLastError();
+        return st == CFEM_ERR_NOMEM ? CFEM_OK : st;
+    }
+    const bool fits = P->arena_used + align256(bytes) <= P->arena_bytes;
+    *out = fits ? P->arena + P->arena_used : nullptr;
+    if (fits) P->arena_used += align256(bytes);
+    return CFEM_OK;
+}
+
 // (Re)copies what the systems hold now, and the solution back.
 static dim3 order_grid(const RowOrder &R) {
     return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(2048, 8192 / R.ns)), (unsigned)R.ns);
@@ -3530,9 +3549,11 @@ static int order_back(const RowOrder &R, cudaStream_t s) {
     return CFEM_OK;
 }
 // The order of d_nodes' Morton keys (one system), or by lowest column, and the
-// copy in it: its pattern, and `what`. On failure nothing is held.
-static int order_build(RowOrder &R, const cfem_linsys *L, const int32_t *nnzb, int ns,
+// copy in it: its pattern, and `what`. On failure, and when there is no memory
+// for it (R.mem null), nothing is held.
+static int order_build(cfem_pcg_plan *P, const cfem_linsys *L, const int32_t *nnzb, int ns,
                        const double *d_nodes, int what, cudaStream_t s) {
+    RowOrder &R = P->ro;
     R.ns = ns;
     R.bs = L[0].bs;
     R.mixed = L[0].mode == CFEM_SOLVE_MIXED;
@@ -3583,13 +3604,18 @@ static int order_build(RowOrder &R, const cfem_linsys *L, const int32_t *nnzb, i
         tmp = take(work, std::max(scan_bytes, sort_bytes));
     };
     hold();
-    CFEM_TRY(tmp_alloc(&base, off, s));
+    CFEM_TRY(rs_alloc(P, &base, off, s));
+    pass();
+    int st = base ? rs_alloc(P, &work, off, s) : CFEM_OK;
+    if (!work) {
+        tmp_free(base, s);
+        R = RowOrder{};
+        return st;
+    }
     R.mem = base;
     hold();
+    pass();
     auto run = [&]() -> int {
-        pass();
-        CFEM_TRY(tmp_alloc(&work, off, s));
-        pass();
         CFEM_CUDA(cudaMemcpyAsync(R.src, src.data(), ns * sizeof(OrderDev), cudaMemcpyHostToDevice, s));
         if (d_nodes) {
             CFEM_CUDA(cudaMemsetAsync(box, 0xff, 3 * 8, s));
@@ -3604,7 +3630,7 @@ static int order_build(RowOrder &R, const cfem_linsys *L, const int32_t *nnzb, i
         CFEM_CUDA(cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, len, R.rp, n + 1, s));
         return order_copy(R, RO_COLS | what, s);
     };
-    const int st = run();
+    st = run();
     tmp_free(work, s);
     if (st != CFEM_OK) {
         tmp_free(R.mem, s);
@@ -3718,9 +3744,13 @@ static bool rs_plan(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     // (PERSISTENT: as many launches as it takes, so that a system's answer does
     // not depend on the others of its batch)
     if (P->waves.size() > RS_MAX_WAVES && P->ctx->scheduler != CFEM_SCHED_PERSISTENT) {
-        int64_t entries = 0;
-        for (int i = 0; i < ns; ++i) entries += nnzb[i];
-        if (P->rs_dense || ns > sms || entries * (int64_t)(2 + bs * bs * ts) > RS_DEAL_BYTES * sms)
+        int64_t entries = 0, rows = 0;
+        for (int i = 0; i < ns; ++i) {
+            entries += nnzb[i];
+            rows += systems[i].n_rows;
+        }
+        if (P->rs_dense || ns > sms || entries * (int64_t)(2 + bs * bs * ts) > RS_DEAL_BYTES * sms ||
+            rows >= INT32_MAX)             // (numbers of the copies' rows and entries)
             return false;
         // one launch, the blocks dealt out one by one to the system whose
         // blocks have the most to do
@@ -3776,19 +3806,20 @@ static void *rs_kernel(int bs, int mode, bool co) {
     return bs == 3 ? (void *)k_resident<double, 3> : (void *)k_resident<double, 1>;
 }
 
-// Memory of a resident plan: from the library's pool, or from the plan's
-// arena (*out null when that is full).
-static int rs_alloc(cfem_pcg_plan *P, char **out, size_t bytes, cudaStream_t s) {
-    if (!P->arena) return tmp_alloc(out, bytes, s);
-    const bool fits = P->arena_used + align256(bytes) <= P->arena_bytes;
-    *out = fits ? P->arena + P->arena_used : nullptr;
-    if (fits) P->arena_used += align256(bytes);
+// A resident plan that is not to be: its memory back, the systems' records
+// as they were.
+static int rs_decline(cfem_pcg_plan *P, cudaStream_t s) {
+    for (char **m : {&P->ws_copy, &P->ws_state, &P->ws_sdata}) {
+        if (!P->arena) tmp_free(*m, s);
+        *m = nullptr;
+    }
+    P->hs.assign(P->n_systems, SysDev{});
     return CFEM_OK;
 }
 
 // Builds the resident plan, or leaves P->resident false (the caller then
 // takes another scheduler) when a block's halo does not fit shared memory
-// or the plan its arena.
+// or there is no memory for the plan.
 static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t *nnzb,
                     cudaStream_t s) {
     cfem_ctx *ctx = P->ctx;
@@ -3838,7 +3869,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     const size_t copy = align256(ns * sizeof(SysDev)) + align256(ctas.size() * sizeof(RsCta)) +
                         align256(list.size() * sizeof(int2)) + perm_bytes + 2 * align256((nslices + 1) * 8) + align256(ctas.size() * 8);
     CFEM_TRY(rs_alloc(P, &P->ws_copy, copy, s));
-    if (!P->ws_copy) return CFEM_OK;
+    if (!P->ws_copy) return rs_decline(P, s);
     size_t oc = 0;
     auto take_c = [&](size_t b) { char *p = P->ws_copy + oc; oc += align256(b); return (void *)p; };
     P->d_sys = (SysDev *)take_c(ns * sizeof(SysDev));
@@ -3867,12 +3898,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
         map_bytes = 0;
         for (const RsCta &c : ctas)
             map_bytes = std::max(map_bytes, rs_map_bytes(hs[c.sys].n, c.rows, hs[c.sys].lsh));
-        if (map_bytes > (size_t)RS_SMEM_MAX) {
-            tmp_free(P->ws_copy, s);
-            P->ws_copy = nullptr;
-            hs.assign(ns, SysDev{});
-            return CFEM_OK;
-        }
+        if (map_bytes > (size_t)RS_SMEM_MAX) return rs_decline(P, s);
     }
     CFEM_CUDA(cudaFuncSetAttribute(k_rs_rank, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
     CFEM_CUDA(cudaFuncSetAttribute(k_rs_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, RS_SMEM_MAX));
@@ -3882,7 +3908,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     char *scan_tmp = nullptr;
     CFEM_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, sizes, soff, nslices + 1, s));
     CFEM_TRY(rs_alloc(P, &scan_tmp, scan_bytes, s));
-    if (!scan_tmp) return CFEM_OK;
+    if (!scan_tmp) return rs_decline(P, s);
     CFEM_CUDA(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, sizes, soff, nslices + 1, s));
     if (!P->arena) tmp_free(scan_tmp, s);
     int64_t total = 0;
@@ -3926,12 +3952,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
         CFEM_TRY(rs_alloc(P, &P->ws_sdata, ubytes + cbytes + align256((size_t)total * bs * bs * ts), s));
         take = P->ws_state && P->ws_sdata;
     }
-    if (!take) {
-        if (!P->arena) tmp_free(P->ws_copy, s);
-        P->ws_copy = P->ws_state = P->ws_sdata = nullptr;
-        hs.assign(ns, SysDev{});
-        return CFEM_OK;
-    }
+    if (!take) return rs_decline(P, s);
     P->resident = true;
     P->persistent = false;
     size_t os = 0;
@@ -4119,16 +4140,15 @@ static int plan_build(cfem_ctx *ctx, const cfem_linsys *systems, int n_systems,
     if (!P->slots &&
         (ctx->scheduler == CFEM_SCHED_AUTO || ctx->scheduler == CFEM_SCHED_PERSISTENT) &&
         rs_plan(P, systems, nnzbs.data())) {
-        int st = CFEM_OK;
         std::vector<cfem_linsys> copies;
         if (P->rs_dealt) {
-            st = order_build(P->ro, systems, nnzbs.data(), n_systems, nullptr, 0, s);
-            if (st == CFEM_OK) copies = order_systems(P->ro, systems);
+            CFEM_TRY(order_build(P, systems, nnzbs.data(), n_systems, nullptr, 0, s));
+            if (P->ro.mem) copies = order_systems(P->ro, systems);
         }
-        if (st == CFEM_OK)
+        if (!P->rs_dealt || P->ro.mem)
             CFEM_TRY(rs_build(P, P->rs_dealt ? copies.data() : systems, nnzbs.data(), s));
         if (P->resident) return CFEM_OK;
-        tmp_free(P->ro.mem, s);           // does not fit: the graph scheduler
+        tmp_free(P->ro.mem, s);           // does not fit, or no memory: the graph scheduler
         P->ro = RowOrder{};
         P->rs_dealt = false;
     }
@@ -5399,14 +5419,16 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         flag = (unsigned *)take((size_t)RS_COPIES * nb * 4);
     };
     lay();
-    CFEM_TRY(tmp_alloc(&mem, off, s));
+    CFEM_TRY(rs_alloc(&P, &mem, off, s));
+    if (!mem) return CFEM_OK;
     lay();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     auto run = [&]() -> int {
         CFEM_CUDA(cudaEventCreate(&e0));
         CFEM_CUDA(cudaEventCreate(&e1));
         CFEM_CUDA(cudaEventRecord(e0, s));
-        CFEM_TRY(order_build(P.ro, &L, &nnzb, 1, d_nodes, RO_V64 | RO_V32 | RO_VEC, s));
+        CFEM_TRY(order_build(&P, &L, &nnzb, 1, d_nodes, RO_V64 | RO_V32 | RO_VEC, s));
+        if (!P.ro.mem) return CFEM_OK;
         const cfem_linsys M = order_systems(P.ro, &L)[0];
         P.hs[0].ainv = ainv;
         P.hs[0].gall = gall;

@@ -216,12 +216,15 @@ CFEM_API int cfem_ctx_trim(cfem_ctx *ctx, uint64_t keep_bytes,
  * (cfem_pcg_slots_*) of 3x3 systems store them in the sliced ELL (1,
  * default; room for rows of up to 96 blocks, the layout built when a
  * system is assigned, a system needing more refused) or in the entry-major
- * copy (0); read when the slots are created. get returns -1 for an unknown
- * parameter. */
+ * copy (0); read when the slots are created. ALLOC_FAIL: fault injection (0
+ * default): the n-th allocation of a resident plan's set-up (1 .. 16) finds
+ * no device memory, and the system is solved as one that the resident kernel
+ * does not take. get returns -1 for an unknown parameter. */
 enum { CFEM_PARAM_T10_WARPS = 1, CFEM_PARAM_P1_THREADS = 2, CFEM_PARAM_GRAPH_ITERS = 3,
        CFEM_PARAM_PDL = 4, CFEM_PARAM_SPMV_STAGE = 5, CFEM_PARAM_BARRIER_TIMEOUT_US = 6,
        CFEM_PARAM_BARRIER_HOLD = 7, CFEM_PARAM_SELL_SORT = 8, CFEM_PARAM_SELL3_LANES = 9,
-       CFEM_PARAM_SELL3_STAGED = 10, CFEM_PARAM_SLOT_SELL3 = 11 };
+       CFEM_PARAM_SELL3_STAGED = 10, CFEM_PARAM_SLOT_SELL3 = 11,
+       CFEM_PARAM_ALLOC_FAIL = 12 };
 CFEM_API int cfem_ctx_set_param(cfem_ctx *ctx, int param, int value);
 CFEM_API int cfem_ctx_get_param(const cfem_ctx *ctx, int param);
 /* Number of kernels this library launched through `ctx` so far. */
