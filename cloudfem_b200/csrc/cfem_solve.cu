@@ -4917,6 +4917,8 @@ static int rs_assign(cfem_pcg_plan *P, int slot, const cfem_linsys *L, int32_t n
         CFEM_CUDA(cudaMemcpyAsync(P->rs_sys + slot, &sub->hs[0], sizeof(SysDev),
                                   cudaMemcpyHostToDevice, w));
         CFEM_CUDA(cudaMemsetAsync(P->rs_st + slot, 0, sizeof(SysState), w));
+        if (slot_runs(P, slot, cfem_pcg_plan::SLOT_GRAPH))   // it ends here
+            CFEM_LAUNCH(k_slot_cancel, 1, 32, 0, w, P->d_st + slot, P->d_bar);
         return CFEM_OK;
     };
     st = put();

@@ -117,3 +117,27 @@ def test_admission_estimates_cover_a_request(torch, precision):
         assert 0 < taken <= r.bytes_estimate() + 64 * 2 ** 20, (kind, taken, r.bytes_estimate())
         eng.release(slot)
         eng.close()
+
+
+def test_resident_system_over_a_running_graph_system(torch):
+    """A slot whose system still runs on the graphs is given to a resident one:
+    later rounds leave the first system's x alone, whatever else the graphs run."""
+    import ctypes
+    from cloudfem_b200 import _native as N
+    rt = N.runtime()
+    arrow, band = _system(ARROW[1], 1, "arrow", 1), _system(2000, 1, "band", 2)
+    eng = _engine(rt, 2, 1, N.SOLVE_FP64)
+    first, other = (_block_system(torch, rt, arrow, 1) for _ in range(2))
+    slot = eng.assign(first, 1e-30, 2000, tag="first")
+    eng.assign(other, 1e-13, 2000, tag="other")
+    second = _block_system(torch, rt, band, 1)
+    ls = second.linsys(N.SOLVE_FP64, 1e-13, 2000)
+    N.check(rt.lib.cfem_pcg_slots_assign(eng.handle, slot, ctypes.byref(ls), rt.stream()))
+    torch.cuda.synchronize()
+    eng.busy[slot] = (second, "second")
+    before = first.x.clone()
+    done = _rounds(eng, ["second", "other"])
+    assert torch.equal(first.x, before)
+    x = _exact(band[0], band[4], band[5], band[6])
+    assert np.linalg.norm(done["second"][0].cpu().numpy() - x) <= 1e-12 * np.linalg.norm(x)
+    eng.close()
