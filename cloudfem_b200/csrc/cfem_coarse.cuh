@@ -264,11 +264,11 @@ k_rc_ac(const SysDev *__restrict__ sys, const float *__restrict__ xl, const uint
 // leaves its unknown out: zero row and column. A chain of nb steps of a few us,
 // mostly the way of flag and rows through L2: 148 pieces took 820 us with a
 // pivot block per piece, 690 with two. Waits are bounded; on expiry *err is
-// set and every block returns.
+// set and every block returns (hold: as if no flag came, CFEM_PARAM_BARRIER_HOLD).
 constexpr int RC_RB = 2 * RM;
 __global__ void __launch_bounds__(RT, 1)
 k_rc_inv(const double *__restrict__ ac, int nm, int nb, double *rowbuf, unsigned *flag,
-         double *__restrict__ out, int *err, unsigned long long timeout_ns) {
+         double *__restrict__ out, int *err, unsigned long long timeout_ns, unsigned hold) {
     extern __shared__ __align__(16) double rc_rows[];     // the block's own rows
     __shared__ double D[RC_RB][RC_RB], d0[RC_RB];
     __shared__ __align__(16) double Dt[RC_RB][RC_RB], Ft[RC_RB][RC_RB];   // [column][row]
@@ -357,7 +357,7 @@ k_rc_inv(const double *__restrict__ ac, int nm, int nb, double *rowbuf, unsigned
             if (t == 0) {
                 const unsigned *f = flag + (me % RS_COPIES) * nb + k;
                 unsigned long long t0 = 0;
-                for (unsigned spin = 0; ld_acquire(f) == 0; ++spin)
+                for (unsigned spin = 0; ld_acquire(f) == 0 || hold; ++spin)
                     if ((spin & 63u) == 63u) {
                         const unsigned long long now = globaltimer();
                         if (t0 == 0) t0 = now;

@@ -64,7 +64,7 @@ __device__ __forceinline__ double2 cocg_row(const uint16_t *cp, const double2 *v
 __global__ void __launch_bounds__(RT, 1)
 k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
                 const RsCta *__restrict__ ctas, int nbytes, double rtol2, int max_iter,
-                unsigned long long timeout_ns) {
+                unsigned long long timeout_ns, unsigned hold) {
     extern __shared__ __align__(128) unsigned char rs_area[];
     __shared__ CocgShared sh;
     const SysDev &S = *sys;
@@ -174,7 +174,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
     });
     if (bad) part[3] = -INFINITY;
     CocgState &st = sh.st;
-    if (!rs_sync<4, true>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, 0u, [&](const double t[4]) {
+    if (!rs_sync<4, true>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, hold, [&](const double t[4]) {
             st.rho = make_double2(t[0], t[1]);
             st.rr = t[2];
             st.bb = t[3];
@@ -213,7 +213,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
             part[1] += pq.y;
         });
         ++epoch;
-        if (!rs_sync<2, false>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, 0u, [&](const double t[4]) {
+        if (!rs_sync<2, false>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, hold, [&](const double t[4]) {
                 const double2 mu = make_double2(t[0], t[1]);
                 const double m2 = mu.x * mu.x + mu.y * mu.y;
                 const double r2 = st.rho.x * st.rho.x + st.rho.y * st.rho.y;
@@ -245,7 +245,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
             part[2] += ri.x * ri.x + ri.y * ri.y;
         }
         ++epoch;
-        if (!rs_sync<3, true>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, 0u, [&](const double t[4]) {
+        if (!rs_sync<3, true>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, hold, [&](const double t[4]) {
                 const double2 rho = make_double2(t[0], t[1]);
                 st.rr = t[2];
                 st.iter += 1;

@@ -4058,7 +4058,7 @@ int cocg_resident(cfem_ctx *ctx, int64_t n, const int32_t *ip, const int32_t *ix
         double rtol2 = rtol * rtol;
         void *args[] = {(void *)&P.d_sys, (void *)&d_st, (void *)&P.d_bar, (void *)&P.d_ctas,
                         (void *)&P.rs_smem, (void *)&rtol2, (void *)&max_iter,
-                        (void *)&P.bar_timeout_ns};
+                        (void *)&P.bar_timeout_ns, (void *)&P.bar_hold};
         CFEM_CUDA(cudaEventRecord(e0, s));
         CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_resident_cocg, dim3((unsigned)P.rs_ctas),
                                               dim3(RT), args, (size_t)P.rs_smem, s));
@@ -5449,7 +5449,7 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         int *err = &P.d_bar->err;
         unsigned long long limit = P.bar_timeout_ns;
         void *args[] = {(void *)&ac, (void *)&inm, (void *)&nb, (void *)&rowbuf, (void *)&flag,
-                        (void *)&ainv, (void *)&err, (void *)&limit};
+                        (void *)&ainv, (void *)&err, (void *)&limit, (void *)&P.bar_hold};
         CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_rc_inv, dim3((unsigned)nb), dim3(RT), args,
                                               inv_bytes, s));
         g_launches.fetch_add(1, std::memory_order_relaxed);

@@ -195,11 +195,11 @@ CFEM_API int cfem_ctx_trim(cfem_ctx *ctx, uint64_t keep_bytes,
  * measured fastest: sliced ELL for FP64 scalar rows and for 3x3 blocks, the
  * staged windows for FP32 scalar rows.
  * BARRIER_TIMEOUT_US: how long (microseconds, 1 .. 60e6; default 4e6) a
- * block of the persistent scheduler waits at its grid barrier before it
- * gives up; the solve then ends with CFEM_ERR_TIMEOUT and the context stays
- * usable. BARRIER_HOLD: fault injection for that path (0 default, or 1):
- * the barrier counts one phantom block that never arrives, so every wait
- * runs to the limit; no other waits of the library are affected. Both are
+ * block of a cooperative launch (persistent and resident kernels, the coarse
+ * inverse) waits for the others before it gives up; the solve then ends with
+ * CFEM_ERR_TIMEOUT and the context stays usable. BARRIER_HOLD: fault injection
+ * for those paths (0 default, or 1): as if one block never arrived, so every
+ * wait runs to the limit; no other waits of the library are affected. Both are
  * read when a solve plan is created. SELL_SORT (SpMV staging 3): 1
  * (default) sorts each window of 256 rows by length before cutting it into
  * slices of 32 (less padding), 0 keeps the rows in order (neighbouring
