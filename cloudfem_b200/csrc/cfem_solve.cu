@@ -5428,7 +5428,6 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
     auto run = [&]() -> int {
         CFEM_CUDA(cudaEventCreate(&e0));
         CFEM_CUDA(cudaEventCreate(&e1));
-        CFEM_CUDA(cudaEventRecord(e0, s));
         CFEM_TRY(order_build(&P, &L, &nnzb, 1, d_nodes, RO_V64 | RO_V32 | RO_VEC, s));
         if (!P.ro.mem) return CFEM_OK;
         const cfem_linsys M = order_systems(P.ro, &L)[0];
@@ -5453,6 +5452,7 @@ static int solve_coarse(cfem_ctx *ctx, const cfem_linsys &L, const double *d_nod
         CFEM_CUDA(cudaLaunchCooperativeKernel((void *)k_rc_inv, dim3((unsigned)nb), dim3(RT), args,
                                               inv_bytes, s));
         g_launches.fetch_add(1, std::memory_order_relaxed);
+        CFEM_CUDA(cudaEventRecord(e0, s));             // kernel_ms: the iterations, as elsewhere
         CFEM_TRY(rs_run(&P, s));
         CFEM_CUDA(cudaEventRecord(e1, s));
         CFEM_TRY(noalloc_result(P.d_st, P.d_bar, stats, s));
