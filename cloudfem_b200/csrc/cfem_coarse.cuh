@@ -26,6 +26,7 @@
 // pieces' geometry, P^T A P by blocks of 6 x 6, and its inverse.
 
 constexpr int RC_NB = 40;            // neighbour pieces accumulated at a time
+constexpr int RC_MIN_ITER = 1000;    // iterations a corrected solve may take at least
 
 // Bounding box of the nodes: doubles mapped to ordered integers, so that the
 // atomics' result does not depend on their order.

@@ -50,6 +50,22 @@ def _timed(torch, dm, vals, b, mask, rtol, max_iter, nodes, repeats=3):
     return r, best, launches
 
 
+def test_no_second_run_to_the_limit(torch):
+    """Coordinates that tell nothing about the part, and a limit that neither
+    solve reaches its target in: 1,000 corrected iterations and 3,000 plain ones
+    (an iteration with the correction takes 1.2 to 1.6 of a plain one: 1.4 to 1.55
+    of the plain call, against 2.2 to 2.6 when both go to the limit)."""
+    from cloudfem_b200 import _native as N
+    rng = np.random.default_rng(1)
+    dm, vals, b, mask = _beam(torch, (60, 4, 4), rng)
+    nodes = torch.from_numpy(rng.random((dm.n_nodes, 3))).to(b.device)
+    rp, plain, _ = _timed(torch, dm, vals, b, mask, 1e-12, 3000, None)
+    rc, with_nodes, _ = _timed(torch, dm, vals, b, mask, 1e-12, 3000, nodes)
+    assert rp.status == rc.status == N.CFEM_ERR_NOT_CONVERGED
+    assert rp.iterations == rc.iterations == 3000
+    assert with_nodes <= 1.9 * plain
+
+
 def test_kernel_ms_is_the_iterations(torch):
     """A handful of iterations: the time reported leaves out the correction's
     set-up, whose inverse alone takes half a millisecond."""
