@@ -3791,7 +3791,7 @@ static int rs_vals(cfem_pcg_plan *P, cudaStream_t s) {
 
 static int rs_copies(cfem_pcg_plan *P, cudaStream_t s) {
     const SysDev &S = P->hs[0];
-    if (P->rs_dealt) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_V32, s));
+    if (P->ro.mem) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_V32, s));
     if (P->rs_ts == 16) return rs_vals<double2, 1>(P, s);
     if (S.mode == CFEM_SOLVE_MIXED) return S.bs == 3 ? rs_vals<float, 3>(P, s) : rs_vals<float, 1>(P, s);
     return S.bs == 3 ? rs_vals<double, 3>(P, s) : rs_vals<double, 1>(P, s);
@@ -5405,6 +5405,12 @@ static int solve_coarse(cfem_ctx *ctx, cfem_linsys L, const double *d_nodes,
     if (nnzb < 2048 || !rs_plan(&P, &L, &nnzb)) return CFEM_OK;
     const int64_t n = L.n_rows;
     const int ncta = P.rs_n[0];
+    // What the largest block needs at the least, with no columns but its own
+    // rows: nothing is copied for a system past that (about 0.6 M nodes in FP64)
+    const int most = (int)((n + ncta - 1) / ncta), lsh = rs_lanes(n, nnzb, 3, ncta);
+    if (rs_meta_bytes(most, lsh) + rs_halo_bytes(most, 3, L.mode == CFEM_SOLVE_MIXED ? 4 : 8) +
+            rs_coarse_bytes(most, ncta) > (size_t)RS_SMEM_MAX - 4096)
+        return CFEM_OK;
     const size_t nm = (size_t)RM * ncta;
     int nb = (ncta * RM + RC_RB - 1) / RC_RB, inm = (int)nm;   // pivot blocks, unknowns
     const bool mixed = L.mode == CFEM_SOLVE_MIXED;
@@ -5433,7 +5439,7 @@ static int solve_coarse(cfem_ctx *ctx, cfem_linsys L, const double *d_nodes,
     auto run = [&]() -> int {
         CFEM_CUDA(cudaEventCreate(&e0));
         CFEM_CUDA(cudaEventCreate(&e1));
-        CFEM_TRY(order_build(&P, &L, &nnzb, 1, d_nodes, RO_V64 | RO_V32 | RO_VEC, s));
+        CFEM_TRY(order_build(&P, &L, &nnzb, 1, d_nodes, RO_VEC, s));   // (values: rs_build, if it fits)
         if (!P.ro.mem) return CFEM_OK;
         const cfem_linsys M = order_systems(P.ro, &L)[0];
         P.hs[0].ainv = ainv;

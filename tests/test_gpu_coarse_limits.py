@@ -66,6 +66,32 @@ def test_no_second_run_to_the_limit(torch):
     assert with_nodes <= 1.9 * plain
 
 
+def test_too_large_a_system_is_not_copied(torch):
+    """900,000 block rows in FP64: the largest block's own rows alone are past
+    shared memory with the correction. Not a launch more than the plain solve."""
+    from cloudfem_b200 import _native as N
+    from cloudfem_b200.device import BlockSystem, pcg
+    rt = N.runtime()
+    n, dev = 900000, rt.device
+    i = torch.arange(n, device=dev)
+    cols = torch.stack([i - 1, i, i + 1], 1)
+    keep = (cols >= 0) & (cols < n)
+    rp = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), keep.sum(1).cumsum(0)]).int()
+    w = torch.where(cols == i[:, None], 1.0, -0.3).double()[keep]
+    vals = (w[:, None, None] * torch.eye(3, dtype=torch.float64, device=dev)).reshape(-1)
+    nodes = torch.rand((n, 3), dtype=torch.float64, device=dev)
+    out = []
+    for nd in (None, nodes):
+        x = torch.zeros(3 * n, dtype=torch.float64, device=dev)
+        s = BlockSystem(rt, n, 3, rp, cols[keep].int(), vals, torch.ones_like(x), x, nodes=nd)
+        before = rt.launches()
+        r = pcg([s], N.SOLVE_FP64, 1e-10, 2000)[0]
+        assert r.status == N.CFEM_OK
+        out.append((rt.launches() - before, x))
+    assert out[0][0] == out[1][0]
+    assert torch.equal(out[0][1], out[1][1])
+
+
 def test_kernel_ms_is_the_iterations(torch):
     """A handful of iterations: the time reported leaves out the correction's
     set-up, whose inverse alone takes half a millisecond."""
