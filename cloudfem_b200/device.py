@@ -417,6 +417,13 @@ class BlockSystem:
         self.keep = keep
         # (n_rows, 3) device coordinates of a 3x3 system's nodes, if known:
         # lets pcg() of the system alone use their rigid-body modes
+        if nodes is not None:
+            torch = _torch()
+            if (nodes.dtype != torch.float64 or tuple(nodes.shape) != (n_rows, 3) or
+                    not nodes.is_contiguous() or nodes.device != vals64.device):
+                raise ValueError(
+                    f"nodes must be a contiguous float64 tensor of shape ({n_rows}, 3) on "
+                    f"{vals64.device}, got {nodes.dtype} {tuple(nodes.shape)} on {nodes.device}")
         self.nodes = nodes
 
     def ensure_fp32(self):
