@@ -172,13 +172,16 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
         part[2] += ri.x * ri.x + ri.y * ri.y;
         part[3] += bi.x * bi.x + bi.y * bi.y;
     });
-    if (bad) part[3] = -INFINITY;
+    // (a zero diagonal: told by the state in global memory, which the grid's sum
+    // orders like the pairs)
+    if (bad) atomicExch(&gst->status, (int)CFEM_ERR_BREAKDOWN);
     CocgState &st = sh.st;
     if (!rs_sync<4, true>(sh, mail, nc, bar, cta, epoch, part, timeout_ns, hold, [&](const double t[4]) {
             st.rho = make_double2(t[0], t[1]);
             st.rr = t[2];
             st.bb = t[3];
-            if (t[3] < 0.0 || !isfinite(t[2])) {
+            st.status = *(volatile int *)&gst->status;
+            if (st.status != CFEM_OK || !isfinite(t[2])) {
                 st.done = 1;
                 st.status = CFEM_ERR_BREAKDOWN;
             } else if (t[2] <= rtol2 * t[3]) {
