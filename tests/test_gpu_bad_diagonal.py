@@ -1,5 +1,6 @@
-"""A row without a diagonal entry ends a resident solve with a breakdown, and
-the statistics of that solve are those of the right-hand side."""
+"""A row without a diagonal entry ends a resident solve with a breakdown
+whatever else the first residual holds, and the statistics of that solve are
+those of the right-hand side."""
 
 import ctypes
 
@@ -41,3 +42,27 @@ def test_complex_system_reports_its_norm(torch, n):
     assert st.status == N.CFEM_ERR_BREAKDOWN and st.iterations == 0
     assert abs(st.bnorm - np.linalg.norm(b)) <= 1e-12 * np.linalg.norm(b)
     assert abs(st.relres - 1.0) <= 1e-12
+
+
+@pytest.mark.parametrize("n", [64, 60000])
+def test_breakdown_beside_an_overflowing_magnitude(torch, n):
+    """Row 0's entry at a Dirichlet DOF is so large that the sum of magnitudes
+    squared overflows, while its residual is that of the others."""
+    from cloudfem_b200 import _native as N
+    from cloudfem_b200.device import BlockSystem, pcg
+    rt = N.runtime()
+    A = sp.diags([np.full(n, 2.0), np.full(n - 1, -0.5), np.full(n - 1, -0.5)], [0, 1, -1]).tolil()
+    A[0, 1] = A[1, 0] = 1e160
+    A[n - 7, n - 7] = 0.0
+    A = A.tocsr()
+    A.eliminate_zeros()
+    A.sort_indices()
+    b = np.ones(n)
+    b[0] = 1e160
+    x = np.zeros(n)
+    x[1] = 1.0
+    fixed = np.zeros(n, dtype=np.uint8)
+    fixed[1] = 1
+    s = BlockSystem(rt, n, 1, *[_up(torch, rt, a) for a in (A.indptr.astype(np.int32),
+                                                            A.indices.astype(np.int32), A.data, b, x, fixed)])
+    assert pcg([s], N.SOLVE_FP64, 1e-12, 500)[0].status == N.CFEM_ERR_BREAKDOWN
