@@ -24,14 +24,6 @@ struct CocgShared {
     int quit, nres, own;
 };
 
-__device__ __forceinline__ double2 c_mul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 c_div(double2 a, double2 b) {
-    const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
-}
-
 // One lane's part of a row: sum of a_j v_j over its slots.
 template <bool SM>
 __device__ __forceinline__ double2 cocg_row(const uint16_t *cp, const double2 *vp, int w,
@@ -53,7 +45,7 @@ __device__ __forceinline__ double2 cocg_row(const uint16_t *cp, const double2 *v
         }
 #pragma unroll
         for (int j = 0; j < U; ++j) {
-            const double2 m = c_mul(a[j], halo[c[j]]);
+            const double2 m = cmul(a[j], halo[c[j]]);
             acc.x += t + j < w ? m.x : 0.0;
             acc.y += t + j < w ? m.y : 0.0;
         }
@@ -160,9 +152,9 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
         const double2 dg = *diag, bi = b[rl];
         const double2 ri = make_double2(bi.x - ax.x, bi.y - ax.y);
         double2 di = make_double2(0.0, 0.0);
-        if (dg.x != 0.0 || dg.y != 0.0) di = c_div(make_double2(1.0, 0.0), dg);
+        if (dg.x != 0.0 || dg.y != 0.0) di = cdiv(make_double2(1.0, 0.0), dg);
         else bad = true;
-        const double2 zi = c_mul(di, ri), rz = c_mul(ri, zi);
+        const double2 zi = cmul(di, ri), rz = cmul(ri, zi);
         r[rl] = ri;
         dinv[rl] = di;
         pair[2 * (r0 + rl)] = zi;
@@ -203,7 +195,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
 #pragma unroll
             for (int k = 0; k < 2; ++k)
                 if (i0 + k * RT < nu) {
-                    const double2 m = c_mul(be, o[k]);
+                    const double2 m = cmul(be, o[k]);
                     halo[rs_swz(i0 + k * RT)] = make_double2(z[k].x + m.x, z[k].y + m.y);
                 }
         }
@@ -211,7 +203,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
         part[0] = part[1] = part[2] = part[3] = 0.0;
         product([&](int rl, double2 qi, const double2 *) {
             q[rl] = qi;
-            const double2 pq = c_mul(halo[rs_swz(own + rl)], qi);
+            const double2 pq = cmul(halo[rs_swz(own + rl)], qi);
             part[0] += pq.x;
             part[1] += pq.y;
         });
@@ -224,7 +216,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
                     st.status = CFEM_ERR_BREAKDOWN;
                     st.done = 1;
                 } else {
-                    st.alpha = c_div(st.rho, mu);
+                    st.alpha = cdiv(st.rho, mu);
                 }
             }))
             return;
@@ -232,13 +224,13 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
         const double2 al = st.alpha;
         part[0] = part[1] = part[2] = part[3] = 0.0;
         for (int i = tid; i < nloc; i += RT) {
-            const double2 pi = halo[rs_swz(own + i)], dx = c_mul(al, pi), dr = c_mul(al, q[i]);
+            const double2 pi = halo[rs_swz(own + i)], dx = cmul(al, pi), dr = cmul(al, q[i]);
             double2 xi = x[i], ri = r[i];
             xi.x += dx.x;
             xi.y += dx.y;
             ri.x -= dr.x;
             ri.y -= dr.y;
-            const double2 zi = c_mul(dinv[i], ri), rz = c_mul(ri, zi);
+            const double2 zi = cmul(dinv[i], ri), rz = cmul(ri, zi);
             x[i] = xi;
             r[i] = ri;
             pair[2 * (r0 + i)] = zi;
@@ -261,7 +253,7 @@ k_resident_cocg(const SysDev *__restrict__ sys, CocgState *gst, GridBar *bar,
                     st.status = CFEM_ERR_NOT_CONVERGED;
                     st.done = 1;
                 } else {
-                    st.beta = c_div(rho, st.rho);
+                    st.beta = cdiv(rho, st.rho);
                     st.rho = rho;
                 }
             }))

@@ -31,18 +31,11 @@ struct CState {
     int iter, status, done, pad;
 };
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) {
     return make_double2(a.x + b.x, a.y + b.y);
 }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) {
     return make_double2(a.x - b.x, a.y - b.y);
-}
-__device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
-    const double d = b.x * b.x + b.y * b.y;
-    return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
 }
 
 // Fixed-order block sum of up to 4 doubles per thread into part[blockIdx].
