@@ -577,7 +577,10 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
     unsigned long long epoch = (unsigned long long)(unsigned)sh.st.pad;
     const int iter0 = sh.st.iter;
     auto adv = [&](const double tot[4]) {
-        if (ph == PH_INIT) sh.st.status = *(volatile int32_t *)&gst[place.x].status;   // a bad diagonal
+        // a bad diagonal: minus infinity among the magnitudes, or NaN where those
+        // overflow as well (a NaN of their own makes the residual's sum one too)
+        if (ph == PH_INIT && (tot[3] < 0.0 || (isnan(tot[3]) && isfinite(tot[0]))))
+            sh.st.status = CFEM_ERR_BREAKDOWN;
         advance(S, &sh.st, bar, ph, tot, cta == 0);
     };
     // Coarse correction: w += R_i^T v for a row's vector v (0 at fixed DOFs);
@@ -952,8 +955,7 @@ k_resident(const SysDev *__restrict__ sys, SysState *gst, GridBar *bar,
             part[0] = rr;
             part[1] = s1;
             part[2] = rz;
-            part[3] = aa;
-            if (bad) atomicExch(&gst[place.x].status, (int)CFEM_ERR_BREAKDOWN);
+            part[3] = bad ? -INFINITY : aa;
             ok = rs_sync<4, true>(sh, S.mail, S.ncta, bar, cta, epoch, part, timeout_ns, hold, adv);
         } else {                              // zero right-hand side
             for (int i = tid; i < nd; i += RT)
