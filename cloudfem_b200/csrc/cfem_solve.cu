@@ -3789,12 +3789,16 @@ static int rs_vals(cfem_pcg_plan *P, cudaStream_t s) {
     return CFEM_OK;
 }
 
-static int rs_copies(cfem_pcg_plan *P, cudaStream_t s) {
+static int rs_fill(cfem_pcg_plan *P, cudaStream_t s) {
     const SysDev &S = P->hs[0];
-    if (P->ro.mem) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_V32, s));
     if (P->rs_ts == 16) return rs_vals<double2, 1>(P, s);
     if (S.mode == CFEM_SOLVE_MIXED) return S.bs == 3 ? rs_vals<float, 3>(P, s) : rs_vals<float, 1>(P, s);
     return S.bs == 3 ? rs_vals<double, 3>(P, s) : rs_vals<double, 1>(P, s);
+}
+
+static int rs_copies(cfem_pcg_plan *P, cudaStream_t s) {
+    if (P->ro.mem) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_V32, s));
+    return rs_fill(P, s);
 }
 
 static void *rs_kernel(int bs, int mode, bool co) {
@@ -3948,6 +3952,8 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     const size_t ubytes = align256(lists * 4), cbytes = align256((size_t)total * 2);
     bool take = umax <= 65535 && fixed <= smem_max;   // else too scattered a pattern
     if (take) {
+        // (values in another row order: copied while the host goes on)
+        if (P->ro.mem) CFEM_TRY(order_copy(P->ro, RO_V64 | RO_V32, s));
         CFEM_TRY(rs_alloc(P, &P->ws_state, state, s));
         CFEM_TRY(rs_alloc(P, &P->ws_sdata, ubytes + cbytes + align256((size_t)total * bs * bs * ts), s));
         take = P->ws_state && P->ws_sdata;
@@ -3993,7 +3999,7 @@ static int rs_build(cfem_pcg_plan *P, const cfem_linsys *systems, const int32_t 
     CFEM_CUDA(cudaFuncSetAttribute(ts == 16 ? (void *)k_resident_cocg
                                               : rs_kernel(bs, mode, P->rs_co),
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
-    return rs_copies(P, s);
+    return rs_fill(P, s);
 }
 
 // One launch of the resident kernel: blocks [first, first + n) of the list.
