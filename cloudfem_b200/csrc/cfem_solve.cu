@@ -1,7 +1,8 @@
 // Batched Jacobi-PCG (replaces spla.spsolve / spla.factorized): phases,
 // schedulers and plans. The resident scheduler, which takes most solves of
-// one or a few systems, is in cfem_resident.cuh; the graph scheduler below
-// takes large batches and solve slots; what neither takes runs as follows.
+// one or a few systems, batches up to 2 MB of matrix per SM and most systems in
+// solve slots, is in cfem_resident.cuh; the graph scheduler below takes larger
+// systems and batches; what neither takes runs as follows.
 //
 // All systems of a batch are solved by ONE cooperative launch (after one
 // ordinary INIT launch). Rows of each system are cut into small chunks
@@ -4736,7 +4737,9 @@ extern "C" int cfem_pcg_solve(cfem_ctx *ctx, const cfem_linsys *systems,
 }
 
 // ---------------------------------------------------------------------------
-// Solve slots: continuous batching at iteration level. A slot plan is a
+// Solve slots: continuous batching at iteration level. A system that the
+// resident kernel takes has a resident plan of its own while it is in a slot
+// (rs_assign, rs_round); for the others a slot plan is a
 // plan of n_slots systems of fixed capacity (rows, nonzero blocks), built
 // from placeholder systems of that size on the host-polled graph scheduler,
 // so its work lists, workspace and captured iteration graphs never change.

@@ -457,7 +457,8 @@ class BlockSystem:
 
 def pcg(systems, mode=N.SOLVE_FP64, rtol=1e-12, max_iter=None,
         reliable_delta=0.0, max_stall=0, history=None):
-    """Solve a batch of BlockSystems in one persistent launch.
+    """Solve a batch of BlockSystems (cfem_pcg_solve; one system with node
+    coordinates: cfem_pcg_solve_nodes).
 
     history: optional list (one device f64 tensor of 2*k entries per
     system) receiving (iteration, relres) at each FP64 residual.
@@ -598,7 +599,9 @@ class SlotEngine:
     together in rounds of 16 CG iterations on the engine's own stream; a
     system assigned between rounds joins the running ones, and a finished
     system frees its slot at once. Systems are BlockSystem objects whose
-    arrays stay alive while they are in a slot."""
+    arrays stay alive while they are in a slot. What a slot holds on the resident
+    kernel is returned to the library's pool when its system finishes or is
+    released."""
 
     def __init__(self, rt, n_slots, bs, mode, max_rows, max_nnzb):
         self.rt = rt

@@ -157,8 +157,8 @@ CFEM_API int cfem_ctx_destroy(cfem_ctx *ctx);
  * GRAPH_POLLED  - the same kernels replayed from plain graphs of 16
  *                 iterations, the host polling convergence once per replay
  *                 (every launch visible to per-launch profilers);
- * AUTO          - the resident kernel where it takes the systems in at most
- *                 four launches, or in one with fewer blocks per system (up
+ * AUTO          - the resident kernel where it takes the systems (and finds
+ *                 device memory for its copies) in at most four launches, or in one with fewer blocks per system (up
  *                 to one system per SM and 2 MB of matrix per SM; a system's
  *                 blocks, and the last bits of its answer, then depend on
  *                 the batch); else PERSISTENT when all row chunks fit in one
@@ -479,8 +479,9 @@ CFEM_API int cfem_pcg_solve(cfem_ctx *ctx, const cfem_linsys *systems,
  * several times fewer iterations on elasticity; the answer meets the same
  * tolerance. Systems it is not for (other block sizes or preconditioners, a
  * history asked for, fewer than 2,048 stored blocks, another scheduler than
- * AUTO, a layout that does not fit) and solves that do not converge with it
- * are those of cfem_pcg_solve. Used by solve_elasticity_* (elastic3d.py:230,
+ * AUTO, a layout or memory that does not suffice) and solves that do not
+ * converge with it in a fourth of max_iter (at least 1,000 iterations) are
+ * those of cfem_pcg_solve. kernel_ms leaves out the correction's set-up. Used by solve_elasticity_* (elastic3d.py:230,
  * elastic_tet10.py:228). Synchronises. */
 CFEM_API int cfem_pcg_solve_nodes(cfem_ctx *ctx, const cfem_linsys *system, const double *d_nodes,
                                   cfem_solve_stats *stats, void *stream);
@@ -494,7 +495,8 @@ CFEM_API int cfem_pcg_solve_nodes(cfem_ctx *ctx, const cfem_linsys *system, cons
  * fixed mask. After changing matrix values in place, call refresh before
  * the next solve. A plan has its own stream, events and workspace: plans of
  * one context may be solved from different host threads at the same time.
- * Destroy waits for the plan's work. */
+ * Create and refresh queue work on the given stream that every later solve,
+ * from whatever stream, comes after. Destroy waits for the plan's work. */
 typedef struct cfem_pcg_plan cfem_pcg_plan;
 CFEM_API int cfem_pcg_plan_create(cfem_ctx *ctx, const cfem_linsys *systems,
                                   int32_t n_systems, void *stream,
@@ -522,7 +524,8 @@ CFEM_API int cfem_pcg_plan_destroy(cfem_pcg_plan *plan);
  * capacity. 3x3 slots size their copy for the sliced-ELL layout by default
  * (CFEM_PARAM_SLOT_SELL3): assign then refuses (CFEM_ERR_INVALID, nothing
  * changed) a system whose layout exceeds the slot's room, which a block row
- * of more than 96 blocks can cause.
+ * of more than 96 blocks can cause. What a slot allocates for a system on the
+ * resident kernel is freed when poll finds it finished and at release.
  * The caller keeps a system's arrays alive
  * while it is in a slot and reads x after poll reports it finished. Each
  * system's scalars and sums are its own, so its iterates do not depend on
